@@ -109,6 +109,10 @@ struct PresState {
   int G = 1, rows = 1, pstride = 1;
   // products
   double *rec_s = nullptr, *rec_b = nullptr;       // FP64 3-force records
+  long long *fx_rec[2] = {nullptr, nullptr};       // fixed-point forms of the FP64 records
+  int *fx_te[2] = {nullptr, nullptr};
+  FxState *fx_state = nullptr;
+  FxSystem fx_sys{};
   double *f6 = nullptr, *v6 = nullptr;             // weakly coupled: 6-stride forces, velocities
   double *v_ss = nullptr, *v_sb = nullptr, *v_bb = nullptr, *v_bs = nullptr;
   double *qpart = nullptr;                         // job partial sums
@@ -1227,6 +1231,11 @@ void pres_free(tfs_solver *s) {
   cudaFree(p->cnt);
   cudaFree(p->st);
   cudaFree(p->qcnt);
+  for (int k = 0; k < 2; ++k) {
+    cudaFree(p->fx_rec[k]);
+    cudaFree(p->fx_te[k]);
+  }
+  cudaFree(p->fx_state);
   cudaFree(p->jobs_dev);
   cudaFree(p->rec_s32);
   cudaFree(p->rec_b32);
@@ -1326,6 +1335,12 @@ QueueJob pres_job(tfs_solver *s, const double *tgt, int n_tgt, double at, const 
   queue_chunking(n_src, s->ns + s->nb, &j.chunk, &j.n_chunks);
   j.partial = partial;
   j.block_done = block_done;
+  const PresState *p = s->pres;
+  FxSource f{};
+  f.set = src == p->rec_s ? 0 : 1;
+  f.rec = p->fx_rec[f.set];
+  f.te = p->fx_te[f.set];
+  fx_job(&j, p->fx_state, p->fx_rec[tgt == p->rec_s ? 0 : 1], f, f, s->ns + s->nb, p->fx_sys.lx_min);
   return j;
 }
 
@@ -1364,6 +1379,25 @@ int pres_alloc(tfs_solver *s) {
     return rc;
   TFS_CUDA(cudaHostAlloc((void **)&p->st_host, sizeof(PresScalars), cudaHostAllocDefault),
            "cudaHostAlloc");
+  if ((rc = alloc_dev((void **)&p->fx_rec[0], 48 * ns)) != TFS_OK ||
+      (rc = alloc_dev((void **)&p->fx_rec[1], 48 * nb)) != TFS_OK ||
+      (rc = alloc_dev((void **)&p->fx_te[0], sizeof(int) * ((ns + 31) / 32))) != TFS_OK ||
+      (rc = alloc_dev((void **)&p->fx_te[1], sizeof(int) * ((nb + 31) / 32))) != TFS_OK ||
+      (rc = alloc_dev((void **)&p->fx_state, sizeof(FxState))) != TFS_OK)
+    return rc;
+  {
+    const FxState fx0{0, 0, {kFxEmpty, kFxEmpty}, 0, {kFxEmpty, kFxEmpty}, 0u};
+    TFS_CUDA(cudaMemcpy(p->fx_state, &fx0, sizeof fx0, cudaMemcpyHostToDevice), "cudaMemcpy");
+    FxSystem &q = p->fx_sys = s->fx_sys;  // the frame and lambda of the solver's particles
+    q.rec[0] = p->rec_s;
+    q.rec[1] = p->rec_b;
+    for (int k = 0; k < 2; ++k) {
+      q.fx[k] = p->fx_rec[k];
+      q.te[k] = p->fx_te[k];
+      q.fd[k] = 3;
+    }
+    q.state = p->fx_state;
+  }
   // the work-queue jobs: seg <- seg (unless weakly coupled), seg <- blob,
   // blob <- blob, blob <- seg, each with its own partials and arrival counters
   const size_t part_s = (size_t)kMaxSplits * 3 * ns, part_b = (size_t)kMaxSplits * 3 * nb;
@@ -1486,6 +1520,8 @@ int pres_operator(tfs_solver *s, int fp32, const double *z, const double *resid,
   }
   if (p->n_jobs > 0) {
     const QueueJob *d64 = it ? p->jobs_it_dev : p->jobs_dev;
+    if (!fp32 && (e = launch_fx_pack(p->fx_sys, s->stream)) != cudaSuccess)
+      return cuda_fail(e, "fixed-point pack kernel");
     const QueueJob *d32 = it ? p->jobs32_it_dev : p->jobs32_dev;
     e = fp32 ? launch_queue(1, s->qtune[1][QK_MBB], Q_BLOB, d32, p->jobs32, p->n_jobs, p->qcnt,
                             s->stream)
@@ -1725,7 +1761,7 @@ int pres_solve(tfs_solver *s, int *iters_out) {
   const bool fp32 = s->cfg.precision == TFS_FP32C;
   const GA g = pres_ga(s);
   int rc;
-  if (fp32 && (rc = ensure_origin(s)) != TFS_OK) return rc;  // the FP32 records' origin
+  if ((rc = ensure_origin(s)) != TFS_OK) return rc;  // the FP32 and fixed-point records' origin
   if ((rc = pres_rhs(s)) != TFS_OK) return rc;
   // ||rhs||; r0 = rhs - A x0 into Q_0 (FP64); beta0 = ||r0||; the warm-start
   // tests (mobility_solver.cpp:2121-2320)
@@ -1815,6 +1851,10 @@ int pres_hook(tfs_solver *s, bool tgt_segs, bool src_segs) {
   pres_hook_pack_kernel<<<(np + 255) / 256, 256, 0, s->stream>>>(a, s->f_segs, s->f_blobs,
                                                                   s->x_blobs, p->rec_s, p->rec_b);
   count_launch();
+  int rc = ensure_origin(s);
+  if (rc != TFS_OK) return rc;
+  cudaError_t fe = launch_fx_pack(p->fx_sys, s->stream);
+  if (fe != cudaSuccess) return cuda_fail(fe, "fixed-point pack kernel");
   const void *tgt = tgt_segs ? (const void *)p->rec_s : (const void *)p->rec_b;
   const void *src = src_segs ? (const void *)p->rec_s : (const void *)p->rec_b;
   int j = -1;

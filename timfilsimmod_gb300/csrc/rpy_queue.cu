@@ -38,8 +38,14 @@ cudaError_t launch_queue(int fp32, int variant, int sources, const QueueJob *job
     return cudaErrorInvalidValue;
   const int nvar = fp32 ? kNumQueueVariantsF32 : kNumQueueVariantsF64;
   if (variant < 0 || variant >= nvar) variant = 0;
-  const QueueVariant var = fp32 ? g_qvariants_f32[variant] : g_qvariants_f64[variant];
-  const QueueFn fn = fp32 ? g_queue_f32[variant][sources] : g_queue_f64[variant][sources];
+  if (!fp32) {
+    if (ev) cudaEventRecord(ev[0], st);
+    const cudaError_t e = launch_fx(variant, sources, jobs, jobs_host, n_jobs, counters, st);
+    if (ev) cudaEventRecord(ev[1], st);
+    return e;
+  }
+  const QueueVariant var = g_qvariants_f32[variant];
+  const QueueFn fn = g_queue_f32[variant][sources];
   const long long units = queue_units(jobs_host, n_jobs, var.block * var.tpt);
   if (units <= 0) return cudaSuccess;
   int resident = 1;

@@ -984,7 +984,7 @@ namespace tfs {
 // (s->swimmer_f, updated in place with the blob repulsion's sums as the
 // reference updates swimmer::f): queued on s->stream with one host wait per
 // refinement cycle and none at the end.
-int compute_velocities_dev(tfs_solver *s, int *gmres_iters) {
+int compute_velocities_dev(tfs_solver *s, int *gmres_iters, bool step) {
   if (s->cfg.nswim != 1) return fail(TFS_EINVAL, "compute_velocities solves one swimmer per solver");
   if (!s->have_refs) return fail(TFS_ESTATE, "set the blob references first");
   int rc;
@@ -999,7 +999,16 @@ int compute_velocities_dev(tfs_solver *s, int *gmres_iters) {
   // v_segs = Mss f_segs, v_blobs = Mbs f_segs (one work-queue launch when
   // both target sets exist)
   if (s->ns > 0 && s->nb > 0) {
-    if ((rc = queue_product(s, QK_SEGSRC)) != TFS_OK) return rc;
+    if (s->cfg.precision == TFS_FP64 && !step) {
+      // M_ss in fixed point, M_bs on the FP64 pipe: one launch of both forms
+      // takes longer than one after the other (1 264 against 1 041 us at 3 587
+      // segments and 1 289 blobs: an FP64 instruction holds the issue port)
+      if ((rc = queue_product(s, QK_MSS)) != TFS_OK) return rc;
+      rc = queue_product(s, QL_MBS_FP64);
+    } else {
+      rc = queue_product(s, s->cfg.precision == TFS_FP64 ? (int)QL_SEGSRC_FP64 : (int)QK_SEGSRC);
+    }
+    if (rc != TFS_OK) return rc;
   } else {
     if ((rc = tfs_evaluate_segment_segment_mobility(s)) != TFS_OK) return rc;
     if ((rc = tfs_evaluate_blob_segment_mobility(s)) != TFS_OK) return rc;
@@ -1011,7 +1020,11 @@ int compute_velocities_dev(tfs_solver *s, int *gmres_iters) {
   int iters = 0;
   if ((rc = linear_solve(s, &iters, early)) != TFS_OK) return rc;
   // v_segs += Msb f_blobs (the solved blob forces)
-  if ((rc = tfs_evaluate_segment_blob_mobility(s)) != TFS_OK) return rc;
+  if (step && s->cfg.precision == TFS_FP64 && s->pres == nullptr && s->ns > 0 && s->nb > 0)
+    rc = queue_product(s, QL_MSB_FP64);
+  else
+    rc = tfs_evaluate_segment_blob_mobility(s);
+  if (rc != TFS_OK) return rc;
   s->last_iters = iters;
   if (gmres_iters) *gmres_iters = iters;
   return TFS_OK;
@@ -1053,7 +1066,7 @@ int tfs_compute_velocities(tfs_solver *s, double *swimmer_f, int *gmres_iters) {
   std::memcpy(s->f6_host, swimmer_f, 8 * 6);
   TFS_CUDA(cudaMemcpyAsync(s->swimmer_f, s->f6_host, 8 * 6, cudaMemcpyHostToDevice, s->stream),
            "copy swimmer force");
-  int rc = compute_velocities_dev(s, gmres_iters);
+  int rc = compute_velocities_dev(s, gmres_iters, false);
   if (rc != TFS_OK) return rc;
   TFS_CUDA(cudaMemcpyAsync(s->f6_host, s->swimmer_f, 8 * 6, cudaMemcpyDeviceToHost, s->stream),
            "read swimmer force");

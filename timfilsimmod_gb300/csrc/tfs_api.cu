@@ -106,6 +106,11 @@ static void free_all(tfs_solver *s) {
   cudaFree(s->rec_blobs);
   cudaFree(s->rec_segs_x2);
   cudaFree(s->rec_blobs_x2);
+  for (int k = 0; k < 2; ++k) {
+    cudaFree(s->fx_rec[k]);
+    cudaFree(s->fx_te[k]);
+  }
+  cudaFree(s->fx_state);
   cudaFree(s->rec_ff);
   cudaFree(s->bar_grid);
   cudaFree(s->wc_z);
@@ -203,7 +208,36 @@ static QueueJob make_job(tfs_solver *s, bool tgt_segs, bool src_segs, bool src_b
   // and arrival counters
   j.partial = s->scratch + (tgt_segs ? (size_t)0 : (size_t)kMaxSplits * 6 * s->ns);
   j.block_done = s->qcount + 2 + (tgt_segs ? 0 : (s->ns + 31) / 32);
+  FxSource seg{}, blob{};
+  seg.rec = s->fx_rec[0];
+  seg.te = s->fx_te[0];
+  seg.set = 0;
+  blob.rec = s->fx_rec[1];
+  blob.te = s->fx_te[1];
+  blob.set = 1;
+  fx_job(&j, s->fx_state, s->fx_rec[tgt_segs ? 0 : 1], src_segs ? seg : blob, blob, s->ns + s->nb,
+         s->fx_sys.lx_min);
   return j;
+}
+
+// The fixed-point form's view of the solver's records.
+static void build_fx_systems(tfs_solver *s) {
+  FxSystem &q = s->fx_sys;
+  const double as = s->cfg.a_seg, ab = s->cfg.a_blob;
+  q.rec[0] = (const double *)s->rec_segs;
+  q.rec[1] = (const double *)s->rec_blobs;
+  q.n[0] = s->ns;
+  q.n[1] = s->nb;
+  q.fd[0] = 6;
+  q.fd[1] = 3;
+  for (int k = 0; k < 2; ++k) {
+    q.fx[k] = s->fx_rec[k];
+    q.te[k] = s->fx_te[k];
+  }
+  q.origin = s->origin;
+  q.lx_min = fx_lambda_exponent(std::min(as, ab), std::min(as, ab));
+  q.lx_max = fx_lambda_exponent(std::max(as, ab), std::max(as, ab));
+  q.state = s->fx_state;
 }
 
 static void add_job(tfs_solver *s, int kind, bool tgt_segs, bool src_segs, bool src_blobs,
@@ -215,7 +249,7 @@ static void add_job(tfs_solver *s, int kind, bool tgt_segs, bool src_segs, bool 
 // Job lists of every launch kind (segment-target jobs first: their pairs cost
 // more), copied to the device once.
 static int build_queue_jobs(tfs_solver *s) {
-  for (int k = 0; k < kNumQueueKinds; ++k) s->qjobs_n[k] = 0;
+  for (int k = 0; k < kNumQueueLists; ++k) s->qjobs_n[k] = 0;
   add_job(s, QK_MSS, true, true, false, OUT_ASSIGN);
   add_job(s, QK_MBS, false, true, false, OUT_ASSIGN);
   add_job(s, QK_SEGSRC, true, true, false, OUT_ASSIGN);
@@ -224,6 +258,20 @@ static int build_queue_jobs(tfs_solver *s) {
   add_job(s, QK_MBB, false, false, true, OUT_ASSIGN);
   add_job(s, QK_GRAND, true, true, true, OUT_ASSIGN);
   add_job(s, QK_GRAND, false, true, true, OUT_ASSIGN);
+  // FP64 sums whose rounding the caller's iteration amplifies stay on the FP64
+  // pipe: the right-hand side of the free-body solve, M_bs (a difference of
+  // 1e-14 in a warm start grows up to 1e5 times in the solution of the FP64
+  // GMRES), and every product of an implicit step (Broyden's iteration carries
+  // 1e-15 in a velocity to 1e-9 in the tether forces)
+  static const int fp64_lists[3][2] = {
+      {QK_MBS, QL_MBS_FP64}, {QK_SEGSRC, QL_SEGSRC_FP64}, {QK_MSB, QL_MSB_FP64}};
+  for (const auto &l : fp64_lists) {
+    s->qjobs_n[l[1]] = s->qjobs_n[l[0]];
+    for (int j = 0; j < s->qjobs_n[l[0]]; ++j) {
+      s->qjobs[l[1]][j] = s->qjobs[l[0]][j];
+      s->qjobs[l[1]][j].fx_state = nullptr;
+    }
+  }
   TFS_CUDA(cudaMemcpy(s->qjobs_dev, s->qjobs, sizeof s->qjobs, cudaMemcpyHostToDevice),
            "copy queue jobs");
   return TFS_OK;
@@ -233,11 +281,15 @@ static int queue_sources(int kind) {
   return kind == QK_GRAND ? Q_SEG_BLOB : (kind == QK_MSB || kind == QK_MBB) ? Q_BLOB : Q_SEG;
 }
 
-int tfs::queue_product(tfs_solver *s, int kind) {
+int tfs::queue_product(tfs_solver *s, int list) {
   const int fp32 = s->cfg.precision == TFS_FP32C;
+  const int kind = list < kNumQueueKinds ? list
+                   : list == QL_MBS_FP64 ? (int)QK_MBS
+                   : list == QL_MSB_FP64 ? (int)QK_MSB
+                                         : (int)QK_SEGSRC;
   const int src = queue_sources(kind);
   int rc;
-  if (fp32 && (rc = ensure_origin(s)) != TFS_OK) return rc;
+  if ((fp32 || list < kNumQueueKinds) && (rc = ensure_origin(s)) != TFS_OK) return rc;
   // the records of both particle kinds: sources, and the targets' positions
   cudaError_t e;
   if (s->ns > 0) {
@@ -248,10 +300,12 @@ int tfs::queue_product(tfs_solver *s, int kind) {
     e = launch_pack(fp32, 3, s->rec_blobs, s->x_blobs, s->f_blobs, s->nb, s->origin, s->stream);
     if (e != cudaSuccess) return cuda_fail(e, "pack kernel");
   }
+  if (!fp32 && list < kNumQueueKinds && (e = launch_fx_pack(s->fx_sys, s->stream)) != cudaSuccess)
+    return cuda_fail(e, "fixed-point pack kernel");
   if (s->product_service != nullptr)  // one launch shared with other swimmers' products
-    return product_service_run(s->product_service, s, kind, fp32, src);
-  e = launch_queue(fp32, s->qtune[fp32][kind], src, s->qjobs_dev + 2 * kind, s->qjobs[kind],
-                   s->qjobs_n[kind], s->qcount, s->stream, next_events(s));
+    return product_service_run(s->product_service, s, list, fp32, src);
+  e = launch_queue(fp32, s->qtune[fp32][kind], src, s->qjobs_dev + 2 * list, s->qjobs[list],
+                   s->qjobs_n[list], s->qcount, s->stream, next_events(s));
   if (e != cudaSuccess) return cuda_fail(e, "RPY work-queue kernel");
   return TFS_OK;
 }
@@ -356,6 +410,11 @@ int tfs_solver_create(const tfs_config *cfg, tfs_solver **out) {
       (rc = alloc_dev(&s->rec_blobs, record_bytes(0, 3) * nb)) ||
       (rc = alloc_dev(&s->rec_segs_x2, 80 * (size_t)ns)) ||
       (rc = alloc_dev(&s->rec_blobs_x2, 48 * (size_t)nb)) ||
+      (rc = alloc_dev((void **)&s->fx_rec[0], 72 * (size_t)ns)) ||
+      (rc = alloc_dev((void **)&s->fx_rec[1], 48 * (size_t)nb)) ||
+      (rc = alloc_dev((void **)&s->fx_te[0], sizeof(int) * ((size_t)(ns + 31) / 32))) ||
+      (rc = alloc_dev((void **)&s->fx_te[1], sizeof(int) * ((size_t)(nb + 31) / 32))) ||
+      (rc = alloc_dev((void **)&s->fx_state, sizeof(FxState))) ||
       (rc = alloc_dev(&s->rec_ff, ff_record_bytes() * nb)) ||
       (rc = alloc_dev(&s->bar_grid, barrier_grid_bytes(ns, nb))) ||
       (rc = alloc_dev((void **)&s->scratch, dsz * s->scratch_elems)) ||
@@ -382,7 +441,10 @@ int tfs_solver_create(const tfs_config *cfg, tfs_solver **out) {
   cudaMemsetAsync(s->origin, 0, dsz * origin_elems(), s->stream);
   cudaMemsetAsync(s->origin_cnt, 0, 2 * sizeof(unsigned), s->stream);
   cudaMemsetAsync(s->qcount, 0, sizeof(unsigned) * qcount_elems, s->stream);
+  const FxState fx0{0, 0, {kFxEmpty, kFxEmpty}, 0, {kFxEmpty, kFxEmpty}, 0u};
+  cudaMemcpyAsync(s->fx_state, &fx0, sizeof fx0, cudaMemcpyHostToDevice, s->stream);
   e = cudaStreamSynchronize(s->stream);
+  build_fx_systems(s);
   if (e == cudaSuccess && (rc = build_queue_jobs(s)) != TFS_OK) {
     free_all(s);
     delete s;
@@ -718,9 +780,16 @@ int tfs_solver_autotune(tfs_solver *s, int precision_mask, int reps) {
   for (int p = 0; p < 2 && rc == TFS_OK; ++p) {
     if (!(precision_mask & (1 << p))) continue;
     s->cfg.precision = p;  // TFS_FP64 = 0, TFS_FP32C = 1
-    if (p == TFS_FP32C && (rc = ensure_origin(s)) != TFS_OK) break;
+    if ((rc = ensure_origin(s)) != TFS_OK) break;
     if (s->ns > 0 && (rc = pack(s, 1)) != TFS_OK) break;
     if (s->nb > 0 && (rc = pack(s, 0)) != TFS_OK) break;
+    if (p == TFS_FP64) {
+      const cudaError_t pe = launch_fx_pack(s->fx_sys, s->stream);
+      if (pe != cudaSuccess) {
+        rc = cuda_fail(pe, "fixed-point pack kernel");
+        break;
+      }
+    }
     if (report.size() > 1) report += ",";
     report += std::string("\"") + (p ? "fp32c" : "fp64") + "\":{";
     bool first_combo = true;
@@ -922,6 +991,6 @@ size_t solver_bytes_estimate(const tfs_config *cfg) {
   const size_t n = 3 * nb + 6, m = std::min<size_t>(350, n);
   const size_t doubles = 15 * ns + 12 * nb + (size_t)kMaxSplits * (6 * ns + 3 * nb) +
                          n * (m + 1) + (m + 1) * (m + 1) + 16 * n + 57 * nb + 256 * (m + 1);
-  return 8 * doubles + 200 * ns + 200 * nb + ((size_t)1 << 20);
+  return 8 * doubles + 273 * ns + 249 * nb + ((size_t)1 << 20);
 }
 }  // namespace tfs

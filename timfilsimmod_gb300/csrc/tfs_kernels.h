@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include "fx_pair.cuh"
+
 namespace tfs {
 
 enum OutMode { OUT_ASSIGN = 0, OUT_ACCUMULATE = 1, OUT_PARTIAL = 2 };
@@ -87,6 +89,38 @@ extern const TileFn g_tile_f64[kNumVariantsF64][kNumCombos];
 // Work-queue products (rpy_queue.cuh): one persistent launch over any number
 // of jobs, each a target set against one or two packed source sets.
 // ---------------------------------------------------------------------------
+// Fixed-point form of FP64 products (rpy_fx.cu). The scales and the verdict
+// of the last fx_pack_kernel: force exponents of the two record arrays, the
+// frame's exponent, and whether the fixed-point form can take the data.
+struct FxState {
+  int ok, Ex, es[2];
+  int bad, es_next[2];  // of the launch under way
+  unsigned arrived;
+};
+constexpr int kFxEmpty = -100000;  // exponent of a set without forces
+// One particle system's records: [0] segments, [1] blobs (n = 0: none).
+struct FxSystem {
+  const double *rec[2];  // packed FP64 records
+  long long *fx[2];      // fixed-point records: 9 (fd = 6) or 6 words each
+  int *te[2];            // force exponents of the tiles of 32
+  int n[2], fd[2];
+  const double *origin;  // the origin kernel's result
+  int lx_min, lx_max;    // of lambda over the pair kinds
+  FxState *state;
+};
+// One source set of a job.
+struct FxSource {
+  const long long *rec;
+  const int *te;
+  int set;         // its FxState::es
+  int lx, tshift;  // lambda = 2^lx; lx - lx_min
+  float near_q;    // (a_i + a_j)^2 / lambda^2, widened
+  fx::Limb s;
+};
+// At most this many chunks: their 12-byte partial sums fit where kMaxSplits
+// 8-byte ones do.
+constexpr int kFxMaxChunks = kMaxSplits * 8 / 12;
+
 struct QueueJob {
   const void *tgt_rec;     // packed records of the targets (their positions are read)
   const void *src_a;       // packed source records, set A
@@ -106,7 +140,11 @@ struct QueueJob {
   int vd;                  // 6 (segment targets) or 3 (blob targets)
   int mode;                // OUT_ASSIGN or OUT_ACCUMULATE
   int chunk, n_chunks;     // sources per unit (a multiple of kQueueQuantum), chunks
-  int pad;
+  // FP64 jobs: the fixed-point form (fx_state null: none)
+  FxState *fx_state;
+  const long long *fx_tgt;
+  FxSource fx[2];
+  int fx_chunk, fx_chunks; // tiles of 32 sources per unit, chunks
 };
 struct QueueArgs {
   const QueueJob *jobs;    // device array, costliest pairs first
@@ -125,7 +163,6 @@ typedef cudaError_t (*QueueFn)(const QueueArgs &, int ctas, cudaStream_t, int *r
 extern const QueueVariant g_qvariants_f32[kNumQueueVariantsF32];
 extern const QueueVariant g_qvariants_f64[kNumQueueVariantsF64];
 extern const QueueFn g_queue_f32[kNumQueueVariantsF32][kNumQueueSources];
-extern const QueueFn g_queue_f64[kNumQueueVariantsF64][kNumQueueSources];
 // Chunks are whole multiples of this many sources (every variant's tile
 // size divides it).
 constexpr int kQueueQuantum = 256;
@@ -144,6 +181,16 @@ void queue_chunking(int n_src, int n_particles, int *chunk, int *n_chunks);
 cudaError_t launch_queue(int fp32, int variant, int sources, const QueueJob *jobs,
                          const QueueJob *jobs_host, int n_jobs, unsigned *counters,
                          cudaStream_t st, cudaEvent_t *ev = nullptr);
+// Fixed-point form (rpy_fx.cu): records and scales of a system from its FP64
+// records; the products of jobs whose systems were packed; a job's fields.
+cudaError_t launch_fx_pack(const FxSystem &q, cudaStream_t st);
+cudaError_t launch_fx(int variant, int sources, const QueueJob *jobs, const QueueJob *jobs_host, int n_jobs,
+                      unsigned *counters, cudaStream_t st);
+int fx_lambda_exponent(double ai, double aj);
+// Fill the job's fixed-point fields (its sizes, radii and records are set);
+// false (and fx_state null) where the radii leave it to FP64.
+bool fx_job(QueueJob *j, FxState *state, const long long *tgt, const FxSource &a, const FxSource &b,
+            int n_particles, int lx_min);
 // Work units of the jobs for a variant's target block (BLOCK * TPT targets).
 long long queue_units(const QueueJob *jobs_host, int n_jobs, int block_targets);
 // The products a solver launches through the queue: M_ss, M_bs, both at once
@@ -151,6 +198,10 @@ long long queue_units(const QueueJob *jobs_host, int n_jobs, int block_targets);
 // mobility (all sources, both target kinds: two jobs).
 enum QueueKind { QK_MSS = 0, QK_MBS = 1, QK_SEGSRC = 2, QK_MSB = 3, QK_MBB = 4, QK_GRAND = 5 };
 constexpr int kNumQueueKinds = 6;
+// The same lists with their jobs kept on the FP64 pipe (tfs_api.cu
+// build_queue_jobs), tuned as QK_MBS, QK_SEGSRC and QK_MSB.
+constexpr int kNumQueueLists = 9;
+enum { QL_MBS_FP64 = 6, QL_SEGSRC_FP64 = 7, QL_MSB_FP64 = 8 };
 
 // Tuning of one launch: variant and the number of full waves (resident CTAs
 // on every SM) the source splitting aims for.

@@ -33,6 +33,11 @@ struct tfs_solver {
   unsigned *origin_cnt = nullptr;  // [2] last-CTA counters of the origin passes
   void *rec_segs = nullptr, *rec_blobs = nullptr;
   void *rec_segs_x2 = nullptr, *rec_blobs_x2 = nullptr;  // FP32x2 records
+  // fixed-point records of FP64 products (rpy_fx.cu)
+  long long *fx_rec[2] = {nullptr, nullptr};
+  int *fx_te[2] = {nullptr, nullptr};
+  tfs::FxState *fx_state = nullptr;
+  tfs::FxSystem fx_sys{};
   void *rec_ff = nullptr;  // float-float blob records (the refinement residual)
   void *bar_grid = nullptr;     // barrier forces: hashed grid of the sources
   double *wc_z = nullptr, *wc_f = nullptr;  // weakly coupled filaments: means, total forces
@@ -105,9 +110,9 @@ struct tfs_solver {
   // built once at creation (host copy and device copy), the launch counters
   // and per-target-block arrival counters, and the tuned variant per
   // (precision, kind)
-  tfs::QueueJob qjobs[tfs::kNumQueueKinds][2];
-  int qjobs_n[tfs::kNumQueueKinds] = {};
-  tfs::QueueJob *qjobs_dev = nullptr;  // [kNumQueueKinds][2]
+  tfs::QueueJob qjobs[tfs::kNumQueueLists][2];
+  int qjobs_n[tfs::kNumQueueLists] = {};
+  tfs::QueueJob *qjobs_dev = nullptr;  // [kNumQueueLists][2]
   unsigned *qcount = nullptr;          // [2] launch counters, then arrival counters
   int qtune[2][tfs::kNumQueueKinds] = {};
   // products shared with other swimmers' (one work-queue launch for all that
@@ -155,8 +160,9 @@ int ensure_origin(tfs_solver *s);
 int pack(tfs_solver *s, int segs);
 TileArgs base_args(tfs_solver *s);
 int product(tfs_solver *s, bool tgt_segs, bool src_segs, bool src_blobs, int mode);
-// One work-queue launch of the given kind (QueueKind) on the solver's stream.
-int queue_product(tfs_solver *s, int kind);
+// One work-queue launch of the given list (QueueKind or QL_*) on the solver's
+// stream.
+int queue_product(tfs_solver *s, int list);
 // Float host arrays: copy n floats to (from) a float64 device array,
 // converting on the device through the solver's float staging buffer.
 int h2d_f32(tfs_solver *s, double *dst, const float *src, size_t n, const char *what);
@@ -178,7 +184,8 @@ int product_service_run(ProductService *sv, tfs_solver *s, int kind, int fp32, i
 void product_service_stats(ProductService *sv, long long *launches, long long *products);
 // compute_velocities on the swimmer force already in s->swimmer_f, queued on
 // s->stream without a host wait at the end (solve.cu).
-int compute_velocities_dev(tfs_solver *s, int *gmres_iters);
+// step: the call is part of an implicit step.
+int compute_velocities_dev(tfs_solver *s, int *gmres_iters, bool step);
 // A new time step begins (the stepper's initial guess): FP32C solvers keep
 // the last step's final solution for the extrapolated warm start of the next
 // step's first solve (solve.cu).

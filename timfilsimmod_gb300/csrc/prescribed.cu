@@ -1333,6 +1333,7 @@ QueueJob pres_job(tfs_solver *s, const double *tgt, int n_tgt, double at, const 
     j.pc32[0][k] = j.pc32[1][k] = (float)q[k];
   }
   queue_chunking(n_src, s->ns + s->nb, &j.chunk, &j.n_chunks);
+  queue_chunking32(n_src, j.n_tgt, &j.chunk32, &j.n_chunks32);
   j.partial = partial;
   j.block_done = block_done;
   const PresState *p = s->pres;

@@ -7,7 +7,7 @@
 // (M_ss with M_bs, M_sb, the grand mobility, ...) is not launched on the
 // swimmer's stream: the swimmer packs its source records there, marks them
 // ready with an event and queues its job list. One waiting thread leads: it
-// takes the pending requests of the same precision and source sets as the
+// takes the pending requests of the same precision, source sets and form as the
 // oldest (those that arrived while the previous launch was being issued), in
 // arrival order, up to kQueueMaxJobs jobs, makes one of the service streams
 // wait for each swimmer's records, copies the jobs (costliest units first)
@@ -39,7 +39,7 @@ namespace tfs {
 struct ProductService {
   struct Req {
     tfs_solver *s;
-    int kind, fp32, src, njobs;
+    int list, fp32, src, njobs;  // list: QueueKind or QL_*
     bool done;
     int rc;
   };
@@ -70,11 +70,12 @@ struct ProductService {
     int n = 0;
     for (Req *r : batch) {
       TFS_CUDA(cudaStreamWaitEvent(stream, r->s->pready_ev, 0), "product service: wait for inputs");
-      for (int j = 0; j < r->njobs; ++j) sl.jobs[n++] = r->s->qjobs[r->kind][j];
+      for (int j = 0; j < r->njobs; ++j) sl.jobs[n++] = r->s->qjobs[r->list][j];
     }
     // costliest units first: longer chunks, and 6-component targets before 3
     std::stable_sort(sl.jobs, sl.jobs + n, [](const QueueJob &a, const QueueJob &b) {
-      return (long)a.chunk * (a.vd == 6 ? 2 : 1) > (long)b.chunk * (b.vd == 6 ? 2 : 1);
+      const long ca = a.plain ? a.chunk : a.chunk32, cb = b.plain ? b.chunk : b.chunk32;
+      return ca * (a.vd == 6 ? 2 : 1) > cb * (b.vd == 6 ? 2 : 1);
     });
     TFS_CUDA(cudaMemcpyAsync(sl.dev_jobs, sl.jobs, sizeof(QueueJob) * n, cudaMemcpyHostToDevice,
                              stream),
@@ -88,8 +89,8 @@ struct ProductService {
     return TFS_OK;
   }
 
-  int run(tfs_solver *s, int kind, int fp32, int src) {
-    Req r{s, kind, fp32, src, s->qjobs_n[kind], false, TFS_OK};
+  int run(tfs_solver *s, int list, int fp32, int src) {
+    Req r{s, list, fp32, src, s->qjobs_n[list], false, TFS_OK};
     if (r.njobs == 0) return TFS_OK;
     TFS_CUDA(cudaEventRecord(s->pready_ev, s->stream), "product service: inputs ready");
     std::unique_lock<std::mutex> g(m);
@@ -107,7 +108,9 @@ struct ProductService {
       const Req *head = pending.front();
       for (auto it = pending.begin(); it != pending.end();) {
         Req *q = *it;
-        if (q->fp32 == head->fp32 && q->src == head->src && jobs + q->njobs <= kQueueMaxJobs) {
+        if (q->fp32 == head->fp32 && q->src == head->src &&
+            (q->list >= kNumQueueKinds) == (head->list >= kNumQueueKinds) &&  // plain or not
+            jobs + q->njobs <= kQueueMaxJobs) {
           jobs += q->njobs;
           batch.push_back(q);
           it = pending.erase(it);
@@ -184,8 +187,8 @@ int product_service_attach(ProductService *sv, tfs_solver *s) {
   return TFS_OK;
 }
 
-int product_service_run(ProductService *sv, tfs_solver *s, int kind, int fp32, int src) {
-  return sv->run(s, kind, fp32, src);
+int product_service_run(ProductService *sv, tfs_solver *s, int list, int fp32, int src) {
+  return sv->run(s, list, fp32, src);
 }
 
 void product_service_stats(ProductService *sv, long long *launches, long long *products) {

@@ -461,13 +461,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) rpy_fx_kernel(const QueueArgs q) 
       if (fixed)
         fx_unit<6, FDA, FDB, BLOCK>(job, blk, c, smem, &s_last);
       else
-        queue_unit<double, 6, FDA, FDB, BLOCK, 1, kFp64Tile>(
+        queue_unit<double, 6, FDA, FDB, BLOCK, 1, kFp64Tile, false>(
             job, blk, c, reinterpret_cast<double *>(smem), nullptr, &s_last);
     } else {
       if (fixed)
         fx_unit<3, FDA, FDB, BLOCK>(job, blk, c, smem, &s_last);
       else
-        queue_unit<double, 3, FDA, FDB, BLOCK, 1, kFp64Tile>(
+        queue_unit<double, 3, FDA, FDB, BLOCK, 1, kFp64Tile, false>(
             job, blk, c, reinterpret_cast<double *>(smem), nullptr, &s_last);
     }
     __syncthreads();

@@ -31,6 +31,7 @@
 
 #include <cuda_runtime.h>
 
+#include "rpy_pair2.cuh"
 #include "rpy_tile.cuh"
 #include "tfs_kernels.h"
 
@@ -68,7 +69,9 @@ __device__ __forceinline__ PairConst<T> job_pair_const(const QueueJob &job, int 
 // as such; the block's last unit adds the pairs of all chunks in chunk
 // order with TwoSum and converts once to FP64, times 1/(8 pi mu). FP64: plain
 // FP64 sums, added in chunk order.
-template <typename T, int VD, int FDA, int FDB, int BLOCK, int TPT, int TS>
+// PACKED (FP32): the packed pair sums of rpy_pair2.cuh and their chunks; else
+// one source after another (rpy_tile.cuh).
+template <typename T, int VD, int FDA, int FDB, int BLOCK, int TPT, int TS, bool PACKED>
 __device__ __forceinline__ void queue_unit(const QueueJob &job, int blk, int c, T *smem,
                                            float *hl, int *s_last) {
   constexpr bool kComp = sizeof(T) == 4;
@@ -93,25 +96,37 @@ __device__ __forceinline__ void queue_unit(const QueueJob &job, int blk, int c, 
   const int warp0 = tile0 + (threadIdx.x & ~31);
   const bool compute = warp0 < n_tgt;
   const int n_src = job.n_a + job.n_b;
-  const int s0 = c * job.chunk;
-  const int s1 = min(s0 + job.chunk, n_src);
+  const int chunk = PACKED ? job.chunk32 : job.chunk, nc = PACKED ? job.n_chunks32 : job.n_chunks;
+  const int s0 = c * chunk;
+  const int s1 = min(s0 + chunk, n_src);
   {
     const PairConst<T> pc = job_pair_const<T>(job, 0);
     const int lo = min(s0, job.n_a), hi = min(s1, job.n_a);
-    if (lo < hi)
-      sum_source_range<T, VD, FDA, BLOCK, TPT, TS>(
-          v, xt, yt, zt, reinterpret_cast<const T *>(job.src_a), lo, hi, pc, smem, hl, compute);
+    if (lo < hi) {
+      if constexpr (PACKED)
+        sum_source_range2<VD, FDA, BLOCK, TPT, TS>(
+            xt, yt, zt, reinterpret_cast<const T *>(job.src_a), lo, hi, pc, smem, hl, compute);
+      else
+        sum_source_range<T, VD, FDA, BLOCK, TPT, TS>(
+            v, xt, yt, zt, reinterpret_cast<const T *>(job.src_a), lo, hi, pc, smem, hl, compute);
+    }
   }
   if constexpr (FDB > 0) {
     const PairConst<T> pc = job_pair_const<T>(job, 1);
     const int lo = max(s0 - job.n_a, 0), hi = max(s1 - job.n_a, 0);
-    if (lo < hi)
-      sum_source_range<T, VD, (FDB > 0 ? FDB : 3), BLOCK, TPT, TS>(
-          v, xt, yt, zt, reinterpret_cast<const T *>(job.src_b), lo, hi, pc, smem, hl, compute);
+    if (lo < hi) {
+      constexpr int FD = FDB > 0 ? FDB : 3;
+      if constexpr (PACKED)
+        sum_source_range2<VD, FD, BLOCK, TPT, TS>(
+            xt, yt, zt, reinterpret_cast<const T *>(job.src_b), lo, hi, pc, smem, hl, compute);
+      else
+        sum_source_range<T, VD, FD, BLOCK, TPT, TS>(
+            v, xt, yt, zt, reinterpret_cast<const T *>(job.src_b), lo, hi, pc, smem, hl, compute);
+    }
   }
 
   const double sc = job.scale;
-  const bool direct = job.n_chunks == 1;
+  const bool direct = nc == 1;
 #pragma unroll
   for (int t = 0; t < TPT; ++t) {
     const int i = tile0 + t * BLOCK + threadIdx.x;
@@ -144,12 +159,11 @@ __device__ __forceinline__ void queue_unit(const QueueJob &job, int blk, int c, 
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    *s_last = atomicAdd(job.block_done + blk, 1u) == (unsigned)(job.n_chunks - 1) ? 1 : 0;
+    *s_last = atomicAdd(job.block_done + blk, 1u) == (unsigned)(nc - 1) ? 1 : 0;
     __threadfence();
   }
   __syncthreads();
   if (*s_last == 0) return;
-  const int nc = job.n_chunks;
   const size_t stride = (size_t)n_tgt * VD;
 #pragma unroll
   for (int t = 0; t < TPT; ++t) {
@@ -162,14 +176,15 @@ __device__ __forceinline__ void queue_unit(const QueueJob &job, int blk, int c, 
 #pragma unroll
       for (int k = 0; k < VD; ++k) H[k] = L[k] = 0.f;
       int cc = 0;
-      for (; cc + 4 <= nc; cc += 4) {  // four chunks' loads in flight, added in order
-        float2 a[4][VD];
+      constexpr int kB = VD == 3 ? 10 : 5;  // chunks' loads in flight, added in order
+      for (; cc + kB <= nc; cc += kB) {
+        float2 a[kB][VD];
 #pragma unroll
-        for (int w = 0; w < 4; ++w)
+        for (int w = 0; w < kB; ++w)
 #pragma unroll
           for (int k = 0; k < VD; ++k) a[w][k] = __ldcg(p + (size_t)(cc + w) * stride + k);
 #pragma unroll
-        for (int w = 0; w < 4; ++w)
+        for (int w = 0; w < kB; ++w)
 #pragma unroll
           for (int k = 0; k < VD; ++k) {
             two_sum(H[k], L[k], a[w][k].x);
@@ -221,7 +236,7 @@ __device__ __forceinline__ void queue_unit(const QueueJob &job, int blk, int c, 
   if (threadIdx.x == 0) job.block_done[blk] = 0u;
 }
 
-template <typename T, int FDA, int FDB, int BLOCK, int TPT, int TS, int MINB>
+template <typename T, int FDA, int FDB, int BLOCK, int TPT, int TS, int MINB, bool PACKED>
 __global__ void __launch_bounds__(BLOCK, MINB) rpy_queue_kernel(const QueueArgs q) {
   constexpr int LA = Rec<T, FDA>::len;
   constexpr int LB = FDB > 0 ? Rec<T, (FDB > 0 ? FDB : 3)>::len : 0;
@@ -239,7 +254,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) rpy_queue_kernel(const QueueArgs 
       const QueueJob &jb = q.jobs[j];
       const bool skip = jb.skip != nullptr && *jb.skip != 0;
       const int nblk = skip ? 0 : (jb.n_tgt + BLOCK * TPT - 1) / (BLOCK * TPT);
-      acc += nblk * jb.n_chunks;
+      acc += nblk * (PACKED ? jb.n_chunks32 : jb.n_chunks);
       s_end[j] = acc;
     }
   }
@@ -262,11 +277,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) rpy_queue_kernel(const QueueArgs 
     }
     const QueueJob &job = q.jobs[lo];
     const int local = u - (lo > 0 ? s_end[lo - 1] : 0);
-    const int blk = local / job.n_chunks, c = local - blk * job.n_chunks;
+    const int nc = PACKED ? job.n_chunks32 : job.n_chunks;
+    const int blk = local / nc, c = local - blk * nc;
     if (job.vd == 6)
-      queue_unit<T, 6, FDA, FDB, BLOCK, TPT, TS>(job, blk, c, smem, hl, &s_last);
+      queue_unit<T, 6, FDA, FDB, BLOCK, TPT, TS, PACKED>(job, blk, c, smem, hl, &s_last);
     else
-      queue_unit<T, 3, FDA, FDB, BLOCK, TPT, TS>(job, blk, c, smem, hl, &s_last);
+      queue_unit<T, 3, FDA, FDB, BLOCK, TPT, TS, PACKED>(job, blk, c, smem, hl, &s_last);
     __syncthreads();  // s_unit and the shared tiles are reused by the next unit
   }
   if (threadIdx.x == 0) {
@@ -290,11 +306,11 @@ constexpr size_t queue_smem_bytes() {
 
 // Launch one instantiation with `ctas` CTAs; with ctas == 0 only report the
 // resident CTAs per SM (cached per device).
-template <typename T, int FDA, int FDB, int BLOCK, int TPT, int TS, int MINB>
+template <typename T, int FDA, int FDB, int BLOCK, int TPT, int TS, int MINB, bool PACKED>
 cudaError_t queue_launch_fn(const QueueArgs &a, int ctas, cudaStream_t st, int *resident) {
   constexpr size_t smem = queue_smem_bytes<T, FDA, FDB, BLOCK, TPT, TS>();
   static std::atomic<int> occupancy[kMaxDevices];
-  auto kern = rpy_queue_kernel<T, FDA, FDB, BLOCK, TPT, TS, MINB>;
+  auto kern = rpy_queue_kernel<T, FDA, FDB, BLOCK, TPT, TS, MINB, PACKED>;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -315,10 +331,10 @@ cudaError_t queue_launch_fn(const QueueArgs &a, int ctas, cudaStream_t st, int *
 
 // One row of a queue dispatch table: the three source specifications in
 // the order of QueueSources.
-#define TFS_QUEUE_ROW(T, B, P, S, M)                                                     \
-  {                                                                                      \
-    queue_launch_fn<T, 6, 0, B, P, S, M>, queue_launch_fn<T, 3, 0, B, P, S, M>,          \
-        queue_launch_fn<T, 6, 3, B, P, S, M>                                             \
+#define TFS_QUEUE_ROW(T, B, P, S, M)                                                       \
+  {                                                                                        \
+    queue_launch_fn<T, 6, 0, B, P, S, M, true>, queue_launch_fn<T, 3, 0, B, P, S, M, true>, \
+        queue_launch_fn<T, 6, 3, B, P, S, M, true>                                         \
   }
 
 }  // namespace tfs

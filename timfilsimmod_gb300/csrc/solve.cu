@@ -999,14 +999,14 @@ int compute_velocities_dev(tfs_solver *s, int *gmres_iters, bool step) {
   // v_segs = Mss f_segs, v_blobs = Mbs f_segs (one work-queue launch when
   // both target sets exist)
   if (s->ns > 0 && s->nb > 0) {
-    if (s->cfg.precision == TFS_FP64 && !step) {
-      // M_ss in fixed point, M_bs on the FP64 pipe: one launch of both forms
-      // takes longer than one after the other (1 264 against 1 041 us at 3 587
-      // segments and 1 289 blobs: an FP64 instruction holds the issue port)
-      if ((rc = queue_product(s, QK_MSS)) != TFS_OK) return rc;
-      rc = queue_product(s, QL_MBS_FP64);
+    if (step) {
+      rc = queue_product(s, QL_SEGSRC_PLAIN);
     } else {
-      rc = queue_product(s, s->cfg.precision == TFS_FP64 ? (int)QL_SEGSRC_FP64 : (int)QK_SEGSRC);
+      // M_ss, then M_bs in the plain form (build_queue_jobs). FP64: one launch
+      // of both forms would take longer (1 264 against 1 041 us at 3 587 segments
+      // and 1 289 blobs: an FP64 instruction holds the issue port).
+      if ((rc = queue_product(s, QK_MSS)) != TFS_OK) return rc;
+      rc = queue_product(s, QL_MBS_PLAIN);
     }
     if (rc != TFS_OK) return rc;
   } else {
@@ -1020,8 +1020,8 @@ int compute_velocities_dev(tfs_solver *s, int *gmres_iters, bool step) {
   int iters = 0;
   if ((rc = linear_solve(s, &iters, early)) != TFS_OK) return rc;
   // v_segs += Msb f_blobs (the solved blob forces)
-  if (step && s->cfg.precision == TFS_FP64 && s->pres == nullptr && s->ns > 0 && s->nb > 0)
-    rc = queue_product(s, QL_MSB_FP64);
+  if (step && s->pres == nullptr && s->ns > 0 && s->nb > 0)
+    rc = queue_product(s, QL_MSB_PLAIN);
   else
     rc = tfs_evaluate_segment_blob_mobility(s);
   if (rc != TFS_OK) return rc;

@@ -204,6 +204,7 @@ static QueueJob make_job(tfs_solver *s, bool tgt_segs, bool src_segs, bool src_b
     }
   }
   queue_chunking(j.n_a + j.n_b, s->ns + s->nb, &j.chunk, &j.n_chunks);
+  queue_chunking32(j.n_a + j.n_b, j.n_tgt, &j.chunk32, &j.n_chunks32);
   // segment-target and blob-target jobs of one launch use disjoint partials
   // and arrival counters
   j.partial = s->scratch + (tgt_segs ? (size_t)0 : (size_t)kMaxSplits * 6 * s->ns);
@@ -258,18 +259,21 @@ static int build_queue_jobs(tfs_solver *s) {
   add_job(s, QK_MBB, false, false, true, OUT_ASSIGN);
   add_job(s, QK_GRAND, true, true, true, OUT_ASSIGN);
   add_job(s, QK_GRAND, false, true, true, OUT_ASSIGN);
-  // FP64 sums whose rounding the caller's iteration amplifies stay on the FP64
-  // pipe: the right-hand side of the free-body solve, M_bs (a difference of
+  // Sums whose rounding the caller's iteration amplifies keep the plain form.
+  // FP64: the right-hand side of the free-body solve, M_bs (a difference of
   // 1e-14 in a warm start grows up to 1e5 times in the solution of the FP64
   // GMRES), and every product of an implicit step (Broyden's iteration carries
-  // 1e-15 in a velocity to 1e-9 in the tether forces)
-  static const int fp64_lists[3][2] = {
-      {QK_MBS, QL_MBS_FP64}, {QK_SEGSRC, QL_SEGSRC_FP64}, {QK_MSB, QL_MSB_FP64}};
-  for (const auto &l : fp64_lists) {
+  // 1e-15 in a velocity to 1e-9 in the tether forces). FP32C the same: 4e-7 in
+  // M_bs is up to 2e-5 in the blob forces, and a swimmer's displacement over a
+  // step is a small difference of its filaments'.
+  static const int plain_lists[3][2] = {
+      {QK_MBS, QL_MBS_PLAIN}, {QK_SEGSRC, QL_SEGSRC_PLAIN}, {QK_MSB, QL_MSB_PLAIN}};
+  for (const auto &l : plain_lists) {
     s->qjobs_n[l[1]] = s->qjobs_n[l[0]];
     for (int j = 0; j < s->qjobs_n[l[0]]; ++j) {
       s->qjobs[l[1]][j] = s->qjobs[l[0]][j];
       s->qjobs[l[1]][j].fx_state = nullptr;
+      s->qjobs[l[1]][j].plain = 1;
     }
   }
   TFS_CUDA(cudaMemcpy(s->qjobs_dev, s->qjobs, sizeof s->qjobs, cudaMemcpyHostToDevice),
@@ -284,8 +288,8 @@ static int queue_sources(int kind) {
 int tfs::queue_product(tfs_solver *s, int list) {
   const int fp32 = s->cfg.precision == TFS_FP32C;
   const int kind = list < kNumQueueKinds ? list
-                   : list == QL_MBS_FP64 ? (int)QK_MBS
-                   : list == QL_MSB_FP64 ? (int)QK_MSB
+                   : list == QL_MBS_PLAIN ? (int)QK_MBS
+                   : list == QL_MSB_PLAIN ? (int)QK_MSB
                                          : (int)QK_SEGSRC;
   const int src = queue_sources(kind);
   int rc;

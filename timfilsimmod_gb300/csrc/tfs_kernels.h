@@ -139,7 +139,12 @@ struct QueueJob {
   int n_tgt, n_a, n_b;
   int vd;                  // 6 (segment targets) or 3 (blob targets)
   int mode;                // OUT_ASSIGN or OUT_ACCUMULATE
-  int chunk, n_chunks;     // sources per unit (a multiple of kQueueQuantum), chunks
+  // sums of one source after another in chunks of kQueueQuantum, of the working
+  // precision: FP64 jobs on the FP64 pipe, FP32 jobs unpacked (every job of
+  // a launch alike)
+  int plain;
+  int chunk, n_chunks;     // plain and FP64: sources per unit (a multiple of kQueueQuantum), chunks
+  int chunk32, n_chunks32; // FP32: sources per unit (a multiple of kQueueQuantum32), chunks
   // FP64 jobs: the fixed-point form (fx_state null: none)
   FxState *fx_state;
   const long long *fx_tgt;
@@ -163,9 +168,12 @@ typedef cudaError_t (*QueueFn)(const QueueArgs &, int ctas, cudaStream_t, int *r
 extern const QueueVariant g_qvariants_f32[kNumQueueVariantsF32];
 extern const QueueVariant g_qvariants_f64[kNumQueueVariantsF64];
 extern const QueueFn g_queue_f32[kNumQueueVariantsF32][kNumQueueSources];
+extern const QueueVariant g_qvariant_f32_plain;
+extern const QueueFn g_queue_f32_plain[kNumQueueSources];
 // Chunks are whole multiples of this many sources (every variant's tile
 // size divides it).
 constexpr int kQueueQuantum = 256;
+constexpr int kQueueQuantum32 = 32;
 // Largest number of jobs one launch may carry (the kernel keeps their unit
 // offsets in shared memory).
 constexpr int kQueueMaxJobs = 256;
@@ -174,6 +182,8 @@ constexpr int kQueueMaxJobs = 256;
 // most kMaxSplits chunks. A function of the sizes alone, so a product is
 // split the same way whatever launch carries it.
 void queue_chunking(int n_src, int n_particles, int *chunk, int *n_chunks);
+// The same for FP32 jobs, from the job's own targets.
+void queue_chunking32(int n_src, int n_tgt, int *chunk, int *n_chunks);
 // Launch the queue kernel of (precision, variant, sources) over the jobs
 // (device array `jobs`; `jobs_host` is the same array on the host, used to
 // size the grid). counters: [2] zeroed unsigned. ev (optional): events
@@ -192,16 +202,15 @@ int fx_lambda_exponent(double ai, double aj);
 bool fx_job(QueueJob *j, FxState *state, const long long *tgt, const FxSource &a, const FxSource &b,
             int n_particles, int lx_min);
 // Work units of the jobs for a variant's target block (BLOCK * TPT targets).
-long long queue_units(const QueueJob *jobs_host, int n_jobs, int block_targets);
+long long queue_units(const QueueJob *jobs_host, int n_jobs, int block_targets);  // FP32 jobs
 // The products a solver launches through the queue: M_ss, M_bs, both at once
 // (segment sources, two jobs), M_sb (accumulating), M_bb, and the grand
 // mobility (all sources, both target kinds: two jobs).
 enum QueueKind { QK_MSS = 0, QK_MBS = 1, QK_SEGSRC = 2, QK_MSB = 3, QK_MBB = 4, QK_GRAND = 5 };
 constexpr int kNumQueueKinds = 6;
-// The same lists with their jobs kept on the FP64 pipe (tfs_api.cu
-// build_queue_jobs), tuned as QK_MBS, QK_SEGSRC and QK_MSB.
+// The same lists with their jobs in the plain form (QueueJob::plain).
 constexpr int kNumQueueLists = 9;
-enum { QL_MBS_FP64 = 6, QL_SEGSRC_FP64 = 7, QL_MSB_FP64 = 8 };
+enum { QL_MBS_PLAIN = 6, QL_SEGSRC_PLAIN = 7, QL_MSB_PLAIN = 8 };
 
 // Tuning of one launch: variant and the number of full waves (resident CTAs
 // on every SM) the source splitting aims for.

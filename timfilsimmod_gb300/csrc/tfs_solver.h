@@ -180,7 +180,7 @@ void service_stats(GmresService *sv, long long *launches, long long *solves);
 ProductService *product_service_create();
 void product_service_destroy(ProductService *sv);
 int product_service_attach(ProductService *sv, tfs_solver *s);
-int product_service_run(ProductService *sv, tfs_solver *s, int kind, int fp32, int src);
+int product_service_run(ProductService *sv, tfs_solver *s, int list, int fp32, int src);
 void product_service_stats(ProductService *sv, long long *launches, long long *products);
 // compute_velocities on the swimmer force already in s->swimmer_f, queued on
 // s->stream without a host wait at the end (solve.cu).

@@ -77,14 +77,39 @@ static cudaError_t launch_body_points(int fp32, void *rec, const double *f_segs,
   return cudaGetLastError();
 }
 
-// Source splits: while the point set fills less than one wave of resident
-// CTAs, split the sources so that the grid does (partials summed in split
-// order by launch_reduce_partials); sources per split a multiple of 64.
+// Source splits. A CTA's time is its share of its SM, so a launch takes as long
+// as the SM with the most CTAs: ceil(ctas splits / SMs) / splits of one CTA's
+// sources (977 CTAs on 152 SMs: 7 with one split, 6.43 with seven; medium
+// swimmer on a 63^3 grid, 3.50 and 3.18 ms). While the point set fills less than
+// one wave of resident CTAs, as many splits as fill it. Each split costs 48 B a
+// point of partial sums, taken as 2% of the launch. Sources per split a
+// multiple of 64.
+static int flow_splits(int ctas, int n_src, long slots, size_t most) {
+  const int cap = (int)std::min({(size_t)kMaxSplits, most, (size_t)std::max(1, n_src / 64)});
+  const int fill = (int)std::max(1L, slots / std::max(1, ctas));
+  if (fill > 1) return std::max(1, std::min(cap, fill));
+  const int sms = num_sms();
+  int best = 1;
+  double cost = 1e30;
+  for (int s = 1; s <= std::min(cap, 8) && n_src / s >= 1024; ++s) {
+    const long c = ((long)ctas * s + sms - 1) / sms;
+    const double t = (double)c / s * (1.0 + 0.02 * (s - 1));
+    if (t < cost) {
+      cost = t;
+      best = s;
+    }
+  }
+  return best;
+}
+
 static cudaError_t launch_flow(FlowArgs a, int fp32, int wall, int variant, double *scratch,
                                size_t scratch_elems, cudaStream_t st) {
   if (a.n_flow <= 0) return cudaSuccess;
   const int nvar = fp32 ? kFlowVariantsF32 : kFlowVariantsF64;
   if (variant < 0 || variant >= nvar) variant = 0;
+  // FP32 index 0: four targets a thread above the wall (57 packed operations a
+  // pair; 100 000 points 2.28 against 2.77 ms), where the points fill the SMs
+  if (fp32 && variant == 0 && wall && a.n_flow >= 512L * num_sms()) variant = 1;
   const FlowVariant var = fp32 ? g_flow_variants_f32[variant] : g_flow_variants_f64[variant];
   const FlowFn fn = fp32 ? g_flow_f32[variant][wall ? 1 : 0] : g_flow_f64[variant][wall ? 1 : 0];
   const int per_cta = var.block * var.tpt;
@@ -94,9 +119,7 @@ static cudaError_t launch_flow(FlowArgs a, int fp32, int wall, int variant, doub
   cudaError_t e = fn(a, dim3(0), st, &resident);
   if (e != cudaSuccess) return e;
   const long slots = (long)resident * num_sms();
-  int splits = (int)std::max(1L, slots / std::max(1, ctas));
-  splits = std::min({splits, kMaxSplits, std::max(1, n_src / 64)});
-  if ((size_t)splits * 3 * a.n_flow > scratch_elems) splits = 1;
+  int splits = flow_splits(ctas, n_src, slots, scratch_elems / (3 * (size_t)a.n_flow));
   int chunk = (n_src + splits - 1) / splits;
   chunk = std::max(64, ((chunk + 63) / 64) * 64);
   splits = std::max(1, (n_src + chunk - 1) / chunk);

@@ -16,6 +16,7 @@
 
 #include <cuda_runtime.h>
 
+#include "rpy_pair2.cuh"
 #include "rpy_tile.cuh"
 
 namespace tfs {
@@ -95,6 +96,104 @@ __device__ __forceinline__ void flow_seg_pair(T *v, T xi, T yi, T zi, T sx, T sy
   }
 }
 
+// The FP32 pair of two staged sources (rpy_pair2.cuh): positive and negative
+// terms have sums of their own. z2 = (zi, zi). The wall's terms with hF =
+// dx F0 + dy F1, K = hF - Rz F2 and D = 2 sz / R^5 (D R^2 = 2 sz / R^3):
+//   image       -(F/R + (R.F) (dx, dy, Rz)/R^3),  R.F = hF + Rz F2
+//   correction  D [ (3 zi K + R^2 F2) (dx, dy) - zi R^2 (F0, F1) ],
+//               D [ 3 zi K Rz + R^2 (hF + zi F2) ]
+// 26 packed operations a segment source (57 above the wall), 18 a point.
+// Bound: the FMA pipe and issue, as rpy_pair2.cuh; 250 047 points around the
+// medium swimmer 4.29 -> 3.50 ms (3.18 with the splits of launch_flow), 100 000
+// points above the wall 3.74 -> 2.28 ms, errors against 64-bit sums unchanged
+// (1.82e-6 and 1.78e-6; 1.88e-5).
+template <int FD, bool WALL>
+__device__ __forceinline__ void flow_pair2(float2 (&v)[3], float2 (&n)[3], float2 dx, float2 dy,
+                                           float2 dz, float2 z2, float2 nz, const float2 (&f)[FD]) {
+  const float2 h2 = fma2(dx, dx, mul2(dy, dy));
+  const float2 r2 = fma2(dz, dz, h2);
+  const float2 rm1 = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+  const float2 rm3 = mul2(mul2(rm1, rm1), rm1);
+  const float2 hF = fma2(dx, f[0], mul2(dy, f[1]));
+  const float2 dF = fma2(dz, f[2], hF);
+  if constexpr (FD == 3) {
+    const float2 w = mul2(rm3, dF);
+    v[0] = fma2(rm1, f[0], fma2(w, dx, v[0]));
+    v[1] = fma2(rm1, f[1], fma2(w, dy, v[1]));
+    v[2] = fma2(rm1, f[2], fma2(w, dz, v[2]));
+  } else {
+    const float2 ex = mul2(rm3, dx), ey = mul2(rm3, dy), ez = mul2(rm3, dz);
+    v[0] = fma2(f[4], ez, fma2(rm1, f[0], fma2(dF, ex, v[0])));
+    v[1] = fma2(f[5], ex, fma2(rm1, f[1], fma2(dF, ey, v[1])));
+    v[2] = fma2(f[3], ey, fma2(rm1, f[2], fma2(dF, ez, v[2])));
+    n[0] = fma2(f[5], ey, n[0]);
+    n[1] = fma2(f[3], ez, n[1]);
+    n[2] = fma2(f[4], ex, n[2]);
+    if constexpr (WALL) {
+      const float2 sz = mul2(both(-1.f), nz);
+      const float2 Rz = add2(z2, sz);
+      const float2 R2 = fma2(Rz, Rz, h2);
+      const float2 Rm1 = make_float2(rsqrt_ftz(R2.x), rsqrt_ftz(R2.y));
+      const float2 Rm2 = mul2(Rm1, Rm1), Rm3 = mul2(Rm1, Rm2);
+      const float2 RF = mul2(Rz, f[2]);
+      const float2 W = mul2(Rm3, add2(hF, RF));
+      n[0] = fma2(Rm1, f[0], fma2(W, dx, n[0]));
+      n[1] = fma2(Rm1, f[1], fma2(W, dy, n[1]));
+      n[2] = fma2(Rm1, f[2], fma2(W, Rz, n[2]));
+      const float2 K3 = mul2(mul2(both(3.f), z2), fma2(both(-1.f), RF, hF));  // 3 zi K
+      const float2 E = mul2(mul2(both(2.f), sz), Rm3);                       // D R^2
+      const float2 D = mul2(E, Rm2);
+      const float2 a = mul2(D, fma2(R2, f[2], K3));
+      const float2 b = mul2(E, z2);
+      v[0] = fma2(a, dx, v[0]);
+      n[0] = fma2(b, f[0], n[0]);
+      v[1] = fma2(a, dy, v[1]);
+      n[1] = fma2(b, f[1], n[1]);
+      v[2] = fma2(mul2(D, K3), Rz, fma2(E, fma2(z2, f[2], hF), v[2]));
+    }
+  }
+}
+
+template <int FD, bool WALL, int BLOCK, int TPT, int TS>
+__device__ __forceinline__ void flow_range2(const float (&xt)[TPT], const float (&yt)[TPT],
+                                            const float (&zt)[TPT], const float *__restrict__ rec,
+                                            int lo, int hi, float *smem, float *hl) {
+  constexpr int W = Pair2<FD>::len;
+  for (int base = lo; base < hi; base += TS) {
+    const int cnt = min(TS, hi - base);
+    __syncthreads();
+    stage_pairs<FD, BLOCK>(rec, base, cnt, smem);
+    __syncthreads();
+    float2 v[TPT][3], n[TPT][3];
+#pragma unroll
+    for (int t = 0; t < TPT; ++t)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[t][k] = n[t][k] = make_float2(0.f, 0.f);
+    const int pairs = (cnt + 1) >> 1;
+#pragma unroll 1
+    for (int p = 0; p < pairs; ++p) {
+      float2 nx, ny, nz, f[FD];
+      load_pair<FD>(smem + p * W, nx, ny, nz, f);
+#pragma unroll
+      for (int t = 0; t < TPT; ++t)
+        flow_pair2<FD, WALL>(v[t], n[t], add2(both(xt[t]), nx), add2(both(yt[t]), ny),
+                             add2(both(zt[t]), nz), both(zt[t]), nz, f);
+    }
+#pragma unroll
+    for (int t = 0; t < TPT; ++t)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        float *hp = hl + ((t * 3 + k) * 2) * BLOCK + threadIdx.x, *lp = hp + BLOCK;
+        float h = *hp, l = *lp;
+        float sum = v[t][k].x + v[t][k].y;
+        if (FD == 6) sum -= n[t][k].x + n[t][k].y;
+        two_sum(h, l, sum);
+        *hp = h;
+        *lp = l;
+      }
+  }
+}
+
 template <typename T, int FD, bool WALL, int BLOCK, int TPT, int TS>
 __device__ __forceinline__ void flow_range(T (&v)[TPT][3], const T (&xt)[TPT], const T (&yt)[TPT],
                                            const T (&zt)[TPT], const T *__restrict__ rec, int lo,
@@ -150,17 +249,25 @@ __global__ void __launch_bounds__(BLOCK) flow_kernel(const FlowArgs a) {
   const int s0 = blockIdx.y * a.chunk, s1 = min(s0 + a.chunk, n_src);
   {
     const int lo = min(s0, a.n_segs), hi = min(s1, a.n_segs);
-    if (lo < hi)
-      flow_range<T, 6, WALL, BLOCK, TPT, TS>(v, xt, yt, zt,
-                                             reinterpret_cast<const T *>(a.rec_segs), lo, hi,
-                                             smem, hl);
+    if (lo < hi) {
+      if constexpr (kComp)
+        flow_range2<6, WALL, BLOCK, TPT, TS>(
+            xt, yt, zt, reinterpret_cast<const float *>(a.rec_segs), lo, hi, smem, hl);
+      else
+        flow_range<T, 6, WALL, BLOCK, TPT, TS>(
+            v, xt, yt, zt, reinterpret_cast<const T *>(a.rec_segs), lo, hi, smem, hl);
+    }
   }
   {
     const int lo = max(s0 - a.n_segs, 0), hi = max(s1 - a.n_segs, 0);
-    if (lo < hi)
-      flow_range<T, 3, false, BLOCK, TPT, TS>(v, xt, yt, zt,
-                                              reinterpret_cast<const T *>(a.rec_points), lo, hi,
-                                              smem, hl);
+    if (lo < hi) {
+      if constexpr (kComp)
+        flow_range2<3, false, BLOCK, TPT, TS>(
+            xt, yt, zt, reinterpret_cast<const float *>(a.rec_points), lo, hi, smem, hl);
+      else
+        flow_range<T, 3, false, BLOCK, TPT, TS>(
+            v, xt, yt, zt, reinterpret_cast<const T *>(a.rec_points), lo, hi, smem, hl);
+    }
   }
 #pragma unroll
   for (int t = 0; t < TPT; ++t) {

@@ -133,6 +133,51 @@ __device__ __forceinline__ void far_pair2(Sum2<VD, FD> &v, float2 dx, float2 dy,
   }
 }
 
+// Stage the records [base, base + cnt) as interleaved pairs; no barrier.
+template <int FD, int BLOCK>
+__device__ __forceinline__ void stage_pairs(const float *__restrict__ rec, int base, int cnt,
+                                            float *smem) {
+  constexpr int L = Rec<float, FD>::len, W = Pair2<FD>::len;
+  for (int j = threadIdx.x; j < cnt; j += BLOCK) {
+    const float4 *q = reinterpret_cast<const float4 *>(rec + (size_t)(base + j) * L);
+    float *o = smem + (j >> 1) * W + (j & 1);
+    const float4 a = __ldg(q), b = __ldg(q + 1);
+    o[0] = -a.x;
+    o[2] = -a.y;
+    o[4] = -a.z;
+    o[6] = a.w;
+    o[8] = b.x;
+    o[10] = b.y;
+    if (FD == 6) {
+      o[12] = b.z;
+      o[14] = b.w;
+      o[16] = __ldg(rec + (size_t)(base + j) * L + 8);
+    }
+  }
+  if ((cnt & 1) && threadIdx.x < FD + 3)  // the odd last source's partner
+    smem[(cnt >> 1) * W + 1 + 2 * threadIdx.x] = threadIdx.x < 3 ? 1e15f : 0.f;
+}
+
+// One pair of staged sources: negated positions, forces (and torques).
+template <int FD>
+__device__ __forceinline__ void load_pair(const float *o, float2 &nx, float2 &ny, float2 &nz,
+                                          float2 (&f)[FD]) {
+  const float4 *q = reinterpret_cast<const float4 *>(o);
+  const float4 a = q[0], b = q[1], c = q[2];
+  nx = make_float2(a.x, a.y);
+  ny = make_float2(a.z, a.w);
+  nz = make_float2(b.x, b.y);
+  f[0] = make_float2(b.z, b.w);
+  f[1] = make_float2(c.x, c.y);
+  f[2] = make_float2(c.z, c.w);
+  if constexpr (FD == 6) {
+    const float4 d = q[3];
+    f[3] = make_float2(d.x, d.y);
+    f[4] = make_float2(d.z, d.w);
+    f[5] = *reinterpret_cast<const float2 *>(q + 4);
+  }
+}
+
 // The sources [lo, hi) of one FP32 record array into the compensated sums of
 // this thread's targets (hl, as Comp<float>). compute = false (warp-uniform):
 // the warp has no target of its own and only helps stage the tiles.
@@ -142,29 +187,12 @@ __device__ __forceinline__ void sum_source_range2(const float (&xt)[TPT], const 
                                                   const float *__restrict__ rec, int lo, int hi,
                                                   const PairConst<float> &pc, float *smem, float *hl,
                                                   bool compute) {
-  constexpr int L = Rec<float, FD>::len, W = Pair2<FD>::len;
+  constexpr int W = Pair2<FD>::len;
   const float2 s = both(pc.s), s3 = both(pc.s3);
   for (int base = lo; base < hi; base += TS) {
     const int cnt = min(TS, hi - base);
     __syncthreads();  // previous tile fully consumed
-    for (int j = threadIdx.x; j < cnt; j += BLOCK) {
-      const float4 *q = reinterpret_cast<const float4 *>(rec + (size_t)(base + j) * L);
-      float *o = smem + (j >> 1) * W + (j & 1);
-      const float4 a = __ldg(q), b = __ldg(q + 1);
-      o[0] = -a.x;
-      o[2] = -a.y;
-      o[4] = -a.z;
-      o[6] = a.w;
-      o[8] = b.x;
-      o[10] = b.y;
-      if (FD == 6) {
-        o[12] = b.z;
-        o[14] = b.w;
-        o[16] = __ldg(rec + (size_t)(base + j) * L + 8);
-      }
-    }
-    if ((cnt & 1) && threadIdx.x < FD + 3)  // the odd last source's partner
-      smem[(cnt >> 1) * W + 1 + 2 * threadIdx.x] = threadIdx.x < 3 ? 1e15f : 0.f;
+    stage_pairs<FD, BLOCK>(rec, base, cnt, smem);
     __syncthreads();
     if (!compute) continue;
     Sum2<VD, FD> v[TPT];
@@ -177,23 +205,13 @@ __device__ __forceinline__ void sum_source_range2(const float (&xt)[TPT], const 
     const int pairs = (cnt + 1) >> 1;
 #pragma unroll 1
     for (int p = 0; p < pairs; ++p) {
-      const float4 *q = reinterpret_cast<const float4 *>(smem + p * W);
-      const float4 a = q[0], b = q[1], c = q[2];
-      float2 f[FD];
-      f[0] = make_float2(b.z, b.w);
-      f[1] = make_float2(c.x, c.y);
-      f[2] = make_float2(c.z, c.w);
-      if constexpr (FD == 6) {
-        const float4 d = q[3];
-        f[3] = make_float2(d.x, d.y);
-        f[4] = make_float2(d.z, d.w);
-        f[5] = *reinterpret_cast<const float2 *>(q + 4);
-      }
+      float2 nx, ny, nz, f[FD];
+      load_pair<FD>(smem + p * W, nx, ny, nz, f);
 #pragma unroll
       for (int t = 0; t < TPT; ++t) {
-        const float2 dx = add2(both(xt[t]), make_float2(a.x, a.y));
-        const float2 dy = add2(both(yt[t]), make_float2(a.z, a.w));
-        const float2 dz = add2(both(zt[t]), make_float2(b.x, b.y));
+        const float2 dx = add2(both(xt[t]), nx);
+        const float2 dy = add2(both(yt[t]), ny);
+        const float2 dz = add2(both(zt[t]), nz);
         const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
         rmin[t] = fminf(rmin[t], fminf(r2.x, r2.y));
         float2 rm1;

@@ -243,6 +243,9 @@ cudaError_t launch_pack_x2(int fd, void *rec, const double *x, const double *f, 
 cudaError_t launch_tile(const TileArgs &a, int vd, int fda, int fdb, TileTuning tune,
                         double *scratch, size_t scratch_elems, int mode, cudaStream_t st,
                         cudaEvent_t *ev = nullptr);
+// rpy_bb64.cu: rpy_tile_kernel<double, 3, 3, 0, ...> of 128-source tiles, bit
+// for bit, for the chunk size, splits, mode and output given.
+cudaError_t launch_bb64(const TileArgs &a, int splits, cudaStream_t st);
 cudaError_t launch_barrier(const BarrierArgs &a, cudaStream_t st);
 // Bytes of BarrierArgs::grid for these sizes.
 size_t barrier_grid_bytes(int num_segs, int num_blobs);

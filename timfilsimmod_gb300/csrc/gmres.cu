@@ -14,6 +14,10 @@
 // convention, stopping when |beta_k| / ||rhs|| <= tol or after
 // min(n, max_iter) steps.
 //
+// A warm-started solve amplifies rounding differences up to 1e5 times, so where
+// a sum's order or a multiply-add's rounding could vary between forms of these
+// kernels it is written out (fma, column_sums).
+//
 // Work split. GB300 issues 2 FP64 FMAs per clock per SM, so the FP64 vector
 // work of an Arnoldi step (~4 k n FMAs at step k) is spread over the SMs: the
 // blobs are cut into G contiguous slices, one CTA each (the last CTA also owns
@@ -104,33 +108,104 @@ __device__ __forceinline__ int slice_row(const GmresArgs &a, const Slice &sl, in
   return r < nblob_rows ? 3 * sl.m0 + r : 3 * a.nb + (r - nblob_rows);
 }
 
-// k dot products <w, Q_i> over this CTA's rows (blob rows only when
-// with_body is false) into part[blockIdx.x * stride + i]. red holds >= 32*64.
-__device__ void block_dots(const GmresArgs &a, const Slice &sl, bool with_body, const double *w,
-                           int k, double *part, int stride, double *red) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int rows = 3 * (sl.m1 - sl.m0) + (with_body && sl.body ? 6 : 0);
-  for (int i = 0; i < k; ++i) {
-    const double *qi = a.Q + (size_t)i * a.n;
-    double v = 0.0;
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-      const int t = slice_row(a, sl, r);
-      v += w[t] * qi[t];
-    }
+// Sums of N columns over a warp: v[j] is this lane's value of column j, and
+// the lanes 32/N * j .. 32/N * j + 32/N - 1 return column j's sum. The tree of
+// a __shfl_down reduction of each column (lane l with l + 16, then l + 8, ...),
+// bit for bit: halving the columns as the lanes halve puts two columns' adds
+// of one level in one instruction, 2 N - 1 (N = 32: 31) FP64 adds for N
+// columns instead of 5 N, and a column's levels wait for N others.
+template <int N>
+__device__ __forceinline__ double column_sums(double (&v)[N]) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) red[wid * 64 + (i & 63)] = v;
-    if ((i & 63) == 63 || i == k - 1) {
-      __syncthreads();
-      const int base = i & ~63;
-      if ((int)threadIdx.x <= i - base) {
-        double t = 0.0;
-        for (int ww = 0; ww < nw; ++ww) t += red[ww * 64 + threadIdx.x];
-        part[(size_t)blockIdx.x * stride + base + threadIdx.x] = t;
+  for (int o = 16, m = N; o > 0; o >>= 1) {
+    if (m > 1) {
+      m >>= 1;
+#pragma unroll
+      for (int j = 0; j < m; ++j) {
+        const bool up = lane & o;
+        const double keep = up ? v[j + m] : v[j], send = up ? v[j] : v[j + m];
+        v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
-      __syncthreads();
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
     }
   }
+  return v[0];
+}
+
+// The Arnoldi kernels run kRowThreads threads over the rows of a slice, in
+// kColGroups groups that take the Krylov columns in turn, kCols at a time.
+constexpr int kRowThreads = 128;
+constexpr int kColGroups = 4;
+constexpr int kCols = 16;
+constexpr int kDotThreads = kRowThreads * kColGroups;
+constexpr int kPass = kCols * kColGroups;  // columns of one pass over the rows
+constexpr int kRowsShared = 512;           // rows of w kept in shared memory
+
+// k dot products <w, Q_i> over this CTA's rows (blob rows only when
+// with_body is false) into part[blockIdx.x * stride + i], by kDotThreads
+// threads. wsh: the first kRowsShared rows of w; red: 4 x kPass.
+__device__ void block_dots(const GmresArgs &a, const Slice &sl, bool with_body, const double *w,
+                           const double *wsh, int k, double *part, int stride, double *red) {
+  const int lane = threadIdx.x & 31, x = threadIdx.x % kRowThreads, group = threadIdx.x / kRowThreads;
+  const int rows = 3 * (sl.m1 - sl.m0) + (with_body && sl.body ? 6 : 0);
+  for (int base = 0; base < k; base += kPass) {
+    const int c0 = base + kCols * group;
+    if (c0 < k) {
+      double v[kCols];
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) v[j] = 0.0;
+      for (int r = x; r < rows; r += kRowThreads) {
+        const int t = slice_row(a, sl, r);
+        const double wt = r < kRowsShared ? wsh[r] : w[t];
+        const double *q = a.Q + (size_t)c0 * a.n + t;
+#pragma unroll
+        for (int j = 0; j < kCols; ++j)
+          if (c0 + j < k) v[j] = fma(wt, q[(size_t)j * a.n], v[j]);
+      }
+      const double t = column_sums<kCols>(v);
+      if ((lane & (32 / kCols - 1)) == 0)
+        red[(x >> 5) * kPass + kCols * group + lane / (32 / kCols)] = t;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < min(kPass, k - base)) {
+      double t = 0.0;
+#pragma unroll
+      for (int ww = 0; ww < kRowThreads / 32; ++ww) t += red[ww * kPass + threadIdx.x];
+      part[(size_t)blockIdx.x * stride + base + threadIdx.x] = t;
+    }
+    __syncthreads();
+  }
+}
+
+// Column i of the CTAs' partial dots, i = i0 .. i0 + 3, summed over the CTAs
+// as warp_sum_strided does; lanes 8 j .. 8 j + 7 return column i0 + j.
+__device__ __forceinline__ double sum_dots(const double *part, int G, int stride, int i0, int k) {
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int c = threadIdx.x & 31; c < G; c += 32)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + j < k) v[j] += __ldcg(part + (size_t)c * stride + i0 + j);
+  return column_sums<4>(v);
+}
+
+// w(t) - sum_i h_i Q_i(t), i in order, the loads of 16 columns in flight.
+__device__ __forceinline__ double project_out(const GmresArgs &a, double wt, const double *h, int k,
+                                              int t) {
+  const double *q = a.Q + t;
+  for (int i0 = 0; i0 < k; i0 += 16) {
+    double qv[16], hv[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      qv[i] = i0 + i < k ? q[(size_t)(i0 + i) * a.n] : 0.0;
+      hv[i] = i0 + i < k ? h[i0 + i] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (i0 + i < k) wt = fma(-hv[i], qv[i], wt);
+  }
+  return wt;
 }
 
 // Last-CTA election: every CTA calls this after writing its partials; it
@@ -181,22 +256,48 @@ __device__ void pack_blob_records(const GmresArgs &a, const double *f, int m) {
   }
 }
 
-// sum over this CTA's blobs of (l_m ; d_m x l_m) into part6[blockIdx.x]
-__device__ void kt_partial(const GmresArgs &a, const Slice &sl, const double *l, double *part6,
-                           double *red, double *sh) {
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  for (int m = sl.m0 + threadIdx.x; m < sl.m1; m += blockDim.x) {
+// This thread's part (x = 0 .. kRowThreads - 1) of the sums over a CTA's blobs
+// of (l_m ; d_m x l_m), summed over its warp into red[6 * warp + k]; l(r) is
+// the value at row r of the slice.
+template <typename L>
+__device__ __forceinline__ void kt_warp_sums(const GmresArgs &a, const Slice &sl, int x, L l,
+                                             double *red) {
+  double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int m = sl.m0 + x; m < sl.m1; m += kRowThreads) {
     const double *d = a.diff + 3 * (size_t)m;
-    const double *v = l + 3 * (size_t)m;
+    const int r = 3 * (m - sl.m0);
+    const double v[3] = {l(r), l(r + 1), l(r + 2)};
     s[0] += v[0];
     s[1] += v[1];
     s[2] += v[2];
-    s[3] += d[1] * v[2] - d[2] * v[1];
-    s[4] += d[2] * v[0] - d[0] * v[2];
-    s[5] += d[0] * v[1] - d[1] * v[0];
+    s[3] += fma(d[1], v[2], -__dmul_rn(d[2], v[1]));
+    s[4] += fma(d[2], v[0], -__dmul_rn(d[0], v[2]));
+    s[5] += fma(d[0], v[1], -__dmul_rn(d[1], v[0]));
   }
-  block_sum_vec<6>(s, red, sh);
-  if (threadIdx.x < 6) part6[6 * blockIdx.x + threadIdx.x] = s[threadIdx.x];
+  const double t = column_sums<8>(s);
+  const int lane = threadIdx.x & 31, c = lane >> 2;
+  if ((lane & 3) == 0 && c < 6) red[6 * (x >> 5) + c] = t;
+}
+
+// The CTA's sums from kt_warp_sums (after a barrier) into part6[blockIdx.x].
+__device__ __forceinline__ void kt_store(double *part6, const double *red) {
+  if (threadIdx.x < 6) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < kRowThreads / 32; ++w) t += red[6 * w + threadIdx.x];
+    part6[6 * blockIdx.x + threadIdx.x] = t;
+  }
+}
+
+// sum over this CTA's blobs of (l_m ; d_m x l_m) into part6[blockIdx.x], in
+// CTAs of kRowThreads threads
+__device__ void kt_partial(const GmresArgs &a, const Slice &sl, const double *l, double *part6,
+                           double *red) {
+  const double *ls = l + 3 * (size_t)sl.m0;
+  __syncthreads();  // red is free
+  kt_warp_sums(a, sl, threadIdx.x, [=](int r) { return ls[r]; }, red);
+  __syncthreads();
+  kt_store(part6, red);
 }
 
 // sum over CTAs (in order) of part6, by the last CTA; result in sh[0..6)
@@ -214,24 +315,46 @@ __device__ void sum_part6(const double *part6, int G, double *sh) {
 // ---------------------------------------------------------------------------
 
 // (1) b = -sum_m (in_m ; d_m x in_m); the last CTA forms the body rows
-//     out_vel = KTKinv b - N in_vel. use_iter: in = Q_{k-1}.
-__global__ void __launch_bounds__(kGT) precond_reduce_kernel(GmresArgs a, const double *in_base,
+//     out_vel = KTKinv b - N in_vel. use_iter: in = Q_{k-1}, which the last
+//     step left unnormalised (k > 1): w / ||w|| first.
+__global__ void __launch_bounds__(kGT) precond_reduce_kernel(GmresArgs a, double *in_base,
                                                              double *out, int use_iter) {
-  __shared__ double red[32 * 8], sh[8];
+  __shared__ double red[32], sh[8], insh[kRowsShared];
   GmresScalars *st = a.st;
   if (use_iter && st->done) return;
-  const double *in = use_iter ? in_base + (size_t)(st->iter - 1) * a.n : in_base;
+  const int k = use_iter ? st->iter : 0;
+  double *in = use_iter ? in_base + (size_t)(k - 1) * a.n : in_base;
   const Slice sl = my_slice(a);
-  kt_partial(a, sl, in, a.part6, red, sh);
+  const int rows = slice_rows(sl);
+  const double qn = k > 1 ? st->qnorm : 1.0;
+  for (int r = threadIdx.x; r < rows; r += kGT) {
+    const int t = slice_row(a, sl, r);
+    double v = in[t];
+    if (k > 1) {
+      v = v / qn;
+      in[t] = v;
+    }
+    if (r < kRowsShared) insh[r] = v;
+  }
+  __syncthreads();
+  kt_warp_sums(a, sl, threadIdx.x,
+               [&](int r) { return r < kRowsShared ? insh[r] : in[3 * (size_t)sl.m0 + r]; }, red);
+  __syncthreads();
+  kt_store(a.part6, red);
   if (!last_cta(a.counters + 0)) return;
   sum_part6(a.part6, gridDim.x, sh);
-  if (threadIdx.x == 0) {
-    double b[6], t1[6], t2[6];
-    for (int k = 0; k < 6; ++k) b[k] = -sh[k];
-    matvec6(t1, a.mats + 36, b);         // rotated KTKinv
-    matvec6(t2, a.mats, in + 3 * a.nb);  // rotated body mobility
-    for (int k = 0; k < 6; ++k) out[3 * a.nb + k] = t1[k] - t2[k];
-    a.counters[0] = 0;
+  if (threadIdx.x < 32) {
+    // lanes 0-5: rows of the rotated KTKinv b; lanes 6-11: of the rotated body
+    // mobility in_vel (the body rows another CTA may just have written)
+    const int lane = threadIdx.x, i = lane % 6;
+    const double *M = a.mats + (lane < 6 ? 36 : 0);
+    double s = 0.0;
+    if (lane < 12)
+      for (int j = 0; j < 6; ++j)
+        s += M[i + 6 * j] * (lane < 6 ? -sh[j] : __ldcg(in + 3 * (size_t)a.nb + j));
+    const double t2 = __shfl_down_sync(0xffffffffu, s, 6);
+    if (lane < 6) out[3 * (size_t)a.nb + lane] = s - t2;
+    if (lane == 0) a.counters[0] = 0;
   }
 }
 
@@ -326,7 +449,7 @@ __global__ void __launch_bounds__(kGT) gmres_residual_kernel(GmresArgs a) {
     q0[3 * (size_t)m + 2] = r2;
     ss[0] += r0 * r0 + r1 * r1 + r2 * r2;
   }
-  kt_partial(a, sl, x, a.part6, red, sh);
+  kt_partial(a, sl, x, a.part6, red);
   block_sum_vec<1>(ss, red, sh);
   if (threadIdx.x == 0) a.part[blockIdx.x] = ss[0];
   if (!last_cta(a.counters + 2)) return;
@@ -385,69 +508,90 @@ __global__ void __launch_bounds__(kGT) gmres_residual_scale_kernel(GmresArgs a) 
 // Arnoldi step k: w = A z into Q_k, CGS2 against Q_0..Q_{k-1}, norm, Givens.
 // ---------------------------------------------------------------------------
 
-// w_blob = M_bb z_lambda - (U + Omega x d_m) (v = M_bb z from the tile
-// kernel); first-pass dots over blob rows; the last CTA adds the body rows
-// w_vel = -sum (z_m ; d_m x z_m) and their dot terms: h1.
-__global__ void __launch_bounds__(kGT) arnoldi_dot1_kernel(GmresArgs a) {
-  __shared__ double red[32 * 64], sh[8];
+// w_blob = M_bb z_lambda - (U + Omega x d_m) (v = M_bb z, or its partial sums
+// over the source splits, added in split order); first-pass dots over blob
+// rows; the last CTA adds the body rows w_vel = -sum (z_m ; d_m x z_m) and
+// their dot terms: h1.
+//
+// These three kernels are chains of waits: FP64 adds at 64 to 78 cycles an SM
+// sub-partition, loads, one last CTA. So the columns' sums are formed side by
+// side (column_sums), all loads of a phase are in flight together, and what
+// is independent runs on other warps. At 642 blobs and 17 columns (averages
+// of two implicit steps): 9.0, 7.8 and 10.0 us; 18.7, 13.7 and 13.0 us with a
+// column after the other.
+__global__ void __launch_bounds__(kDotThreads) arnoldi_dot1_kernel(GmresArgs a,
+                                                                   const double *v, int splits) {
+  __shared__ double red[4 * kPass], kred[32], sh[8], wsh[kRowsShared];
   GmresScalars *st = a.st;
   if (st->done) return;
   const int k = st->iter, n = a.n, vel = 3 * a.nb;
   const Slice sl = my_slice(a);
   double *w = a.Q + (size_t)k * n;
   const double *z = a.z;
-  const double u0 = z[vel], u1 = z[vel + 1], u2 = z[vel + 2];
-  const double w0 = z[vel + 3], w1 = z[vel + 4], w2 = z[vel + 5];
-  for (int m = sl.m0 + threadIdx.x; m < sl.m1; m += blockDim.x) {
-    const double *d = a.diff + 3 * (size_t)m;
-    const double *v = a.v + 3 * (size_t)m;
-    w[3 * (size_t)m] = -(u0 - d[1] * w2 + d[2] * w1) + v[0];
-    w[3 * (size_t)m + 1] = -(u1 - d[2] * w0 + d[0] * w2) + v[1];
-    w[3 * (size_t)m + 2] = -(u2 - d[0] * w1 + d[1] * w0) + v[2];
+  const int x = threadIdx.x % kRowThreads, group = threadIdx.x / kRowThreads;
+  if (group == 0) {
+    for (int r = x; r < 3 * (sl.m1 - sl.m0); r += kRowThreads) {
+      const int t = 3 * sl.m0 + r, c = r % 3, c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+      const double *d = a.diff + (t - c);
+      double vt = splits > 1 ? 0.0 : v[t];
+      if (splits > 1)
+#pragma unroll 8
+        for (int p = 0; p < splits; ++p) vt += v[(size_t)p * vel + t];
+      const double wt = -(z[vel + c] - d[c1] * z[vel + 3 + c2] + d[c2] * z[vel + 3 + c1]) + vt;
+      w[t] = wt;
+      if (r < kRowsShared) wsh[r] = wt;
+    }
+  } else if (group == 1) {
+    kt_warp_sums(a, sl, x, [&](int r) { return z[3 * (size_t)sl.m0 + r]; }, kred);
   }
-  kt_partial(a, sl, z, a.part6, red, sh);
   __syncthreads();
-  block_dots(a, sl, false, w, k, a.part, a.part_stride, red);
+  kt_store(a.part6, kred);
+  block_dots(a, sl, false, w, wsh, k, a.part, a.part_stride, red);
   if (!last_cta(a.counters + 3)) return;
   sum_part6(a.part6, gridDim.x, sh);
   if (threadIdx.x < 6) w[vel + threadIdx.x] = -sh[threadIdx.x];
-  __syncthreads();
-  for (int i = threadIdx.x >> 5; i < k; i += blockDim.x >> 5) {
-    double t = warp_sum_strided(a.part + i, gridDim.x, a.part_stride);
-    if ((threadIdx.x & 31) == 0) {
-      const double *qi = a.Q + (size_t)i * n;
-      for (int j = 0; j < 6; ++j) t += w[vel + j] * qi[vel + j];
-      a.h1[i] = t;
-    }
+  const int lane = threadIdx.x & 31;
+  for (int i0 = 4 * (threadIdx.x >> 5); i0 < k; i0 += 4 * (kDotThreads / 32)) {
+    const int i = i0 + (lane >> 3);
+    double q[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) q[j] = i < k ? a.Q[(size_t)i * n + vel + j] : 0.0;
+    double t = sum_dots(a.part, gridDim.x, a.part_stride, i0, k);
+#pragma unroll
+    for (int j = 0; j < 6; ++j) t = fma(-sh[j], q[j], t);
+    if ((lane & 7) == 0 && i < k) a.h1[i] = t;
   }
   if (threadIdx.x == 0) a.counters[3] = 0;
 }
 
 // w -= sum_i h1_i Q_i (this CTA's rows), then second-pass dots: h2, and
 // H(:, k-1) = h1 + h2.
-__global__ void __launch_bounds__(kGT) arnoldi_dot2_kernel(GmresArgs a) {
-  __shared__ double red[32 * 64];
+__global__ void __launch_bounds__(kDotThreads) arnoldi_dot2_kernel(GmresArgs a) {
+  __shared__ double red[4 * kPass], wsh[kRowsShared];
   GmresScalars *st = a.st;
   if (st->done) return;
   const int k = st->iter, n = a.n;
   const Slice sl = my_slice(a);
   double *w = a.Q + (size_t)k * n;
   const int rows = slice_rows(sl);
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+  // rows of 128 threads; four groups share long slices
+  for (int r = threadIdx.x; r < rows; r += kDotThreads) {
     const int t = slice_row(a, sl, r);
-    double wt = w[t];
-    for (int i = 0; i < k; ++i) wt -= a.h1[i] * a.Q[(size_t)i * n + t];
+    const double wt = project_out(a, w[t], a.h1, k, t);
     w[t] = wt;
+    if (r < kRowsShared) wsh[r] = wt;
   }
   __syncthreads();
-  block_dots(a, sl, true, w, k, a.part, a.part_stride, red);
+  block_dots(a, sl, true, w, wsh, k, a.part, a.part_stride, red);
   if (!last_cta(a.counters + 4)) return;
-  const int ld = a.max_iter + 1;
-  for (int i = threadIdx.x >> 5; i < k; i += blockDim.x >> 5) {
-    const double t = warp_sum_strided(a.part + i, gridDim.x, a.part_stride);
-    if ((threadIdx.x & 31) == 0) {
+  const int ld = a.max_iter + 1, lane = threadIdx.x & 31;
+  for (int i0 = 4 * (threadIdx.x >> 5); i0 < k; i0 += 4 * (kDotThreads / 32)) {
+    const int i = i0 + (lane >> 3);
+    const double h1 = i < k ? a.h1[i] : 0.0;
+    const double t = sum_dots(a.part, gridDim.x, a.part_stride, i0, k);
+    if ((lane & 7) == 0 && i < k) {
       a.h2[i] = t;
-      a.H[i + (size_t)(k - 1) * ld] = a.h1[i] + t;
+      a.H[i + (size_t)(k - 1) * ld] = h1 + t;
     }
   }
   if (threadIdx.x == 0) a.counters[4] = 0;
@@ -455,8 +599,15 @@ __global__ void __launch_bounds__(kGT) arnoldi_dot2_kernel(GmresArgs a) {
 
 // w -= sum_i h2_i Q_i, ||w||; the last CTA applies the Givens rotations
 // (mobility_solver.cpp:2370-2413), tests convergence and, when finishing,
-// back-solves for y (:2419-2438).
-__global__ void __launch_bounds__(kGT) arnoldi_norm_kernel(GmresArgs a) {
+// back-solves for y (:2419-2438). The next step's preconditioner divides w by
+// ||w||.
+//
+// A fifth warp turns the column of H by the earlier rotations meanwhile: that
+// needs no norm. What is left after the last CTA's election is a chain of two
+// square roots and three divisions, each of them about a microsecond.
+__global__ void __launch_bounds__(kGT + 32) arnoldi_norm_kernel(GmresArgs a) {
+  extern __shared__ double hsh[];  // cs (then the turned column), sn, the column of H and
+                                   // its turned entries: max_iter + 1 each
   __shared__ double red[32 * 8], sh[8];
   GmresScalars *st = a.st;
   if (st->done) return;
@@ -464,85 +615,101 @@ __global__ void __launch_bounds__(kGT) arnoldi_norm_kernel(GmresArgs a) {
   const Slice sl = my_slice(a);
   double *w = a.Q + (size_t)k * n;
   const int rows = slice_rows(sl);
+  const int ld = a.max_iter + 1;
+  double *H = a.H, *cs = hsh, *sn = hsh + ld, *col = hsh + 2 * ld, *beta = a.beta;
+#define HH(i, j) H[(i) + (size_t)(j) * ld]
   double ss[1] = {0.0};
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-    const int t = slice_row(a, sl, r);
-    double wt = w[t];
-    for (int i = 0; i < k; ++i) wt -= a.h2[i] * a.Q[(size_t)i * n + t];
-    w[t] = wt;
-    ss[0] += wt * wt;
+  if (threadIdx.x >= kGT) {
+    const int lane = threadIdx.x & 31;
+    for (int i = lane; i < k; i += 32) {
+      cs[i] = i < k - 1 ? a.cs[i] : 0.0;
+      sn[i] = i < k - 1 ? a.sn[i] : 0.0;
+      col[i] = HH(i, k - 1);
+    }
+    __syncwarp();
+    // entry i turned by rotation i - 1, before rotation i
+    double h = col[0];
+    for (int i = 1; i < k; ++i) {
+      const double h1 = fma(cs[i - 1], col[i], -__dmul_rn(sn[i - 1], h));
+      if (lane == 0) hsh[3 * ld + i - 1] = h;
+      h = h1;
+    }
+    if (lane == 0) hsh[3 * ld + k - 1] = h;
+    __syncwarp();
+    // the finished entries, in place of the rotations' cosines
+    for (int i = lane; i < k - 1; i += 32)
+      cs[i] = fma(cs[i], hsh[3 * ld + i], __dmul_rn(sn[i], col[i + 1]));
+    if (lane == 0) cs[k - 1] = h;
+  } else {
+    for (int r = threadIdx.x; r < rows; r += kGT) {
+      const int t = slice_row(a, sl, r);
+      const double wt = project_out(a, w[t], a.h2, k, t);
+      w[t] = wt;
+      ss[0] += wt * wt;
+    }
   }
   block_sum_vec<1>(ss, red, sh);
   if (threadIdx.x == 0) a.part[blockIdx.x] = ss[0];
   if (!last_cta(a.counters + 5)) return;
   const double tsum = threadIdx.x < 32 ? warp_sum_strided(a.part, gridDim.x, 1) : 0.0;
+  __shared__ bool finish;
   if (threadIdx.x == 0) {
     const double t = tsum;
     const double qn = sqrt(t);
     st->qnorm = qn;
-    const int ld = a.max_iter + 1;
-    double *H = a.H, *cs = a.cs, *sn = a.sn, *beta = a.beta;
-#define HH(i, j) H[(i) + (size_t)(j) * ld]
-    HH(k, k - 1) = qn;
-    for (int i = 1; i < k; ++i) {
-      const double tt = cs[i - 1] * HH(i - 1, k - 1) + sn[i - 1] * HH(i, k - 1);
-      HH(i, k - 1) = cs[i - 1] * HH(i, k - 1) - sn[i - 1] * HH(i - 1, k - 1);
-      HH(i - 1, k - 1) = tt;
-    }
-    const double hd = HH(k - 1, k - 1), hs = HH(k, k - 1);
+    const double hd = cs[k - 1], hs = qn;
+    double c, s;
     if (hs == 0.0) {
-      cs[k - 1] = 1.0;
-      sn[k - 1] = 0.0;
+      c = 1.0;
+      s = 0.0;
     } else if (fabs(hs) > fabs(hd)) {
       const double tt = hd / hs;
-      sn[k - 1] = (2.0 * (double)(hs > 0) - 1.0) / sqrt(1.0 + tt * tt);
-      cs[k - 1] = tt * sn[k - 1];
+      s = (2.0 * (double)(hs > 0) - 1.0) / sqrt(1.0 + tt * tt);
+      c = tt * s;
     } else {
       const double tt = hs / hd;
-      cs[k - 1] = (2.0 * (double)(hd > 0) - 1.0) / sqrt(1.0 + tt * tt);
-      sn[k - 1] = tt * cs[k - 1];
+      c = (2.0 * (double)(hd > 0) - 1.0) / sqrt(1.0 + tt * tt);
+      s = tt * c;
     }
-    HH(k - 1, k - 1) = cs[k - 1] * hd + sn[k - 1] * hs;
+    a.cs[k - 1] = c;
+    a.sn[k - 1] = s;
+    cs[k - 1] = fma(c, hd, __dmul_rn(s, hs));
     HH(k, k - 1) = 0.0;
-    beta[k] = -sn[k - 1] * beta[k - 1];
-    beta[k - 1] = cs[k - 1] * beta[k - 1];
-    const double rel = fabs(beta[k]) / st->norm_rhs;
+    const double b = beta[k - 1];
+    const double bk = -s * b;
+    beta[k] = bk;
+    beta[k - 1] = c * b;
+    const double rel = fabs(bk) / st->norm_rhs;
     st->rel = rel;
-    bool finish = rel <= a.tol || k == a.max_iter;
+    finish = rel <= a.tol || k == a.max_iter;
     if (!(rel == rel)) {  // NaN: stop and report
       finish = true;
       st->status = 1;
     }
-    if (finish) {
-      double *y = a.y;
-      y[k - 1] = beta[k - 1] / HH(k - 1, k - 1);
-      for (int i = k - 2; i >= 0; --i) {
-        double yi = beta[i];
-        for (int j = k - 1; j > i; --j) yi -= HH(i, j) * y[j];
-        y[i] = yi / HH(i, i);
-      }
-      st->iters = k;
-      st->done = 1;
-    } else {
-      st->iter = k + 1;
-    }
-#undef HH
     a.counters[5] = 0;
   }
-}
-
-// Q_k = w / ||w|| (the step was not the last one).
-__global__ void __launch_bounds__(kGT) arnoldi_scale_kernel(GmresArgs a) {
-  GmresScalars *st = a.st;
-  if (st->done) return;
-  const int k = st->iter - 1, n = a.n;
-  const Slice sl = my_slice(a);
-  double *w = a.Q + (size_t)k * n;
-  const double qn = st->qnorm;
-  const int rows = slice_rows(sl);
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-    const int t = slice_row(a, sl, r);
-    w[t] = w[t] / qn;
+  __syncthreads();
+  for (int i = threadIdx.x; i < k; i += blockDim.x) HH(i, k - 1) = cs[i];
+  if (!finish) {
+    if (threadIdx.x == 0) st->iter = k + 1;
+    return;
+  }
+  // y: from the last row up, each y_j taken out of the rows above at once
+  double *y = col;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) y[i] = beta[i];
+  for (int j = k - 1; j >= 0; --j) {
+    __syncthreads();
+    if (threadIdx.x == 0) y[j] = y[j] / HH(j, j);
+    __syncthreads();
+    const double yj = y[j];
+    for (int i = threadIdx.x; i < j; i += blockDim.x) y[i] = fma(-HH(i, j), yj, y[i]);
+  }
+#undef HH
+  __syncthreads();
+  for (int i = threadIdx.x; i < k; i += blockDim.x) a.y[i] = y[i];
+  if (threadIdx.x == 0) {
+    st->iters = k;
+    st->done = 1;
   }
 }
 
@@ -607,7 +774,7 @@ __global__ void __launch_bounds__(kGT) refine_residual_kernel(GmresArgs a, const
       ss[1] += b[j] * b[j];
     }
   }
-  kt_partial(a, sl, x, a.part6, red, sh);
+  kt_partial(a, sl, x, a.part6, red);
   block_sum_vec<2>(ss, red, sh);
   if (threadIdx.x == 0) {
     a.part[2 * blockIdx.x] = ss[0];
@@ -676,7 +843,7 @@ __global__ void __launch_bounds__(kGT) rhs_kernel(GmresArgs a, const double *fre
   const Slice sl = my_slice(a);
   const int vel = 3 * a.nb;
   for (int t = 3 * sl.m0 + threadIdx.x; t < 3 * sl.m1; t += blockDim.x) rhs[t] = -v_blobs[t];
-  kt_partial(a, sl, frep, a.part6, red, sh);
+  kt_partial(a, sl, frep, a.part6, red);
   if (!last_cta(a.counters + 7)) return;
   sum_part6(a.part6, gridDim.x, sh);
   if (threadIdx.x < 6) {
@@ -701,7 +868,7 @@ __global__ void unit_rhs_kernel(double *rhs, int n, int j) {
 // are latency-bound (a few grid-wide reductions per Arnoldi step); fewer CTAs
 // shorten each last-CTA reduction and leave SMs to other swimmers' streams
 // (measured on GB300: 32 blobs per CTA beats 4 by ~20% per step for 642 and
-// 2562 blobs, results unchanged).
+// 2562 blobs).
 int gmres_grid(int nb, int sms, int *blobs_per_cta) {
   int G = std::max(1, std::min(sms, (nb + 31) / 32));
   int per = std::max(1, (nb + G - 1) / G);
@@ -729,14 +896,13 @@ cudaError_t launch_gmres_precond(const GmresArgs &a, cudaStream_t st) {
   count_launch();
   return cudaGetLastError();
 }
-cudaError_t launch_gmres_arnoldi(const GmresArgs &a, cudaStream_t st) {
-  arnoldi_dot1_kernel<<<a.G, kGT, 0, st>>>(a);
+cudaError_t launch_gmres_arnoldi(const GmresArgs &a, const double *v, int splits,
+                                 cudaStream_t st) {
+  arnoldi_dot1_kernel<<<a.G, kDotThreads, 0, st>>>(a, v, splits);
   count_launch();
-  arnoldi_dot2_kernel<<<a.G, kGT, 0, st>>>(a);
+  arnoldi_dot2_kernel<<<a.G, kDotThreads, 0, st>>>(a);
   count_launch();
-  arnoldi_norm_kernel<<<a.G, kGT, 0, st>>>(a);
-  count_launch();
-  arnoldi_scale_kernel<<<a.G, kGT, 0, st>>>(a);
+  arnoldi_norm_kernel<<<a.G, kGT + 32, 4 * 8 * (a.max_iter + 1), st>>>(a);
   count_launch();
   return cudaGetLastError();
 }

@@ -112,7 +112,9 @@ cudaError_t launch_gmres_finish(const GmresArgs &a, cudaStream_t st);
 cudaError_t launch_gmres_start(const GmresArgs &a, cudaStream_t st);
 cudaError_t launch_gmres_residual(const GmresArgs &a, cudaStream_t st);
 cudaError_t launch_gmres_precond(const GmresArgs &a, cudaStream_t st);
-cudaError_t launch_gmres_arnoldi(const GmresArgs &a, cudaStream_t st);
+// v: M_bb z, or its `splits` partial sums [split][3 nb].
+cudaError_t launch_gmres_arnoldi(const GmresArgs &a, const double *v, int splits,
+                                 cudaStream_t st);
 cudaError_t launch_refine_residual(const GmresArgs &a, const double *x, double *r, double *dx,
                                    int outer, cudaStream_t st);
 cudaError_t launch_axpy(double *x, const double *d, int n, cudaStream_t st);

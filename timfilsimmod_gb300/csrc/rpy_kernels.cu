@@ -484,7 +484,7 @@ static int choose_splits(int ctas, int n_src, int resident, int waves, int ts) {
 
 cudaError_t launch_tile(const TileArgs &a_in, int vd, int fda, int fdb, TileTuning tune,
                         double *scratch, size_t scratch_elems, int mode, cudaStream_t st,
-                        cudaEvent_t *ev) {
+                        cudaEvent_t *ev, int *partials) {
   TileArgs a = a_in;
   const int combo = combo_of(vd, fda, fdb);
   if (combo < 0) return cudaErrorInvalidValue;
@@ -512,6 +512,7 @@ cudaError_t launch_tile(const TileArgs &a_in, int vd, int fda, int fdb, TileTuni
   chunk = ((chunk + kMinChunk - 1) / kMinChunk) * kMinChunk;
   if (chunk == 0) chunk = kMinChunk;
   splits = std::max(1, (n_src + chunk - 1) / chunk);
+  if (partials) *partials = splits;
   a.chunk = chunk;
   const dim3 grid(ctas, splits);
   // the same sums, split further and faster at every size (rpy_bb64.cu: 184 -> 34 us
@@ -532,7 +533,7 @@ cudaError_t launch_tile(const TileArgs &a_in, int vd, int fda, int fdb, TileTuni
   e = bb64 ? launch_bb64(a, splits, st) : fn(a, grid, st, nullptr);
   count_launch();
   if (ev) cudaEventRecord(ev[1], st);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || partials) return e;
   const int n_elems = a.n_tgt * vd;
   reduce_partials_kernel<<<(n_elems + 255) / 256, 256, 0, st>>>(
       final_out, scratch, n_elems, splits, mode == OUT_ACCUMULATE ? 1 : 0, a.skip);

@@ -147,8 +147,8 @@ GmresArgs gmres_args(tfs_solver *s, const double *rhs, double *f_blobs, double *
 }
 
 // v = M_bb (the blob records just packed), in FP64 or FP32C; skipped when
-// *skip is set.
-int mbb_product(tfs_solver *s, int fp32, const int *skip) {
+// *skip is set. partials: as for launch_tile.
+int mbb_product(tfs_solver *s, int fp32, const int *skip, int *partials = nullptr) {
   TileArgs a = base_args(s);
   a.fp32 = fp32;
   a.x_tgt = s->x_blobs;
@@ -161,7 +161,7 @@ int mbb_product(tfs_solver *s, int fp32, const int *skip) {
   a.out = s->vtmp;
   a.skip = skip;
   cudaError_t e = launch_tile(a, 3, 3, 0, s->tune[fp32][C_BB], s->scratch, s->scratch_elems,
-                              OUT_ASSIGN, s->stream);
+                              OUT_ASSIGN, s->stream, nullptr, partials);
   if (e != cudaSuccess) return cuda_fail(e, "blob-blob product");
   return TFS_OK;
 }
@@ -196,8 +196,11 @@ int launch_chunk(tfs_solver *s, const GmresArgs &g, int fp32) {
   for (int k = 0; k < s->chunk; ++k) {
     if ((e = launch_gmres_precond(g, s->stream)) != cudaSuccess)
       return cuda_fail(e, "gmres preconditioner");
-    if ((rc = mbb_product(s, fp32, &s->gst->done)) != TFS_OK) return rc;
-    if ((e = launch_gmres_arnoldi(g, s->stream)) != cudaSuccess) return cuda_fail(e, "gmres arnoldi");
+    int splits = 1;
+    if ((rc = mbb_product(s, fp32, &s->gst->done, &splits)) != TFS_OK) return rc;
+    if ((e = launch_gmres_arnoldi(g, splits > 1 ? s->scratch : s->vtmp, splits, s->stream)) !=
+        cudaSuccess)
+      return cuda_fail(e, "gmres arnoldi");
   }
   return TFS_OK;
 }

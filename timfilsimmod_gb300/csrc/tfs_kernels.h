@@ -240,9 +240,12 @@ cudaError_t launch_pack_x2(int fd, void *rec, const double *x, const double *f, 
 // split launches (the launcher falls back to one split when it is smaller).
 // ev (optional): a pair of events recorded around the tile kernel itself
 // (not the pack or reduce kernels), for the dominant-kernel timing hook.
+// partials (optional): receives the number of splits; with more than one, the
+// partial sums [split][target][vd] stay in scratch for the caller to add in
+// split order.
 cudaError_t launch_tile(const TileArgs &a, int vd, int fda, int fdb, TileTuning tune,
                         double *scratch, size_t scratch_elems, int mode, cudaStream_t st,
-                        cudaEvent_t *ev = nullptr);
+                        cudaEvent_t *ev = nullptr, int *partials = nullptr);
 // rpy_bb64.cu: rpy_tile_kernel<double, 3, 3, 0, ...> of 128-source tiles, bit
 // for bit, for the chunk size, splits, mode and output given.
 cudaError_t launch_bb64(const TileArgs &a, int splits, cudaStream_t st);

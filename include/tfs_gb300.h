@@ -454,11 +454,11 @@ int tfs_stepper_write_files(tfs_stepper *st, int nt, const char *prefix, int bac
  * no state on the device: a swimmer's result is the same alone (a batch of
  * one) and in a batch. The inner GMRES solves of FP32C instances can run
  * in shared cooperative launches of the persistent kernel (in the server,
- * and in a batch unless tfs_batch_share_inner_solves says otherwise): a solve
- * waiting for
- * the GPU is gathered with the others waiting (up to the SM count of CTAs),
- * each on a fixed number of CTAs chosen from its own blob count (about one
- * per 64 blobs), so its arithmetic does not depend on the others. FP32C
+ * and in a batch unless tfs_batch_share_inner_solves says otherwise): up to
+ * four launches run side by side, and a solve that has to wait for them is
+ * gathered with the others waiting (up to the SM count of CTAs), each on a
+ * fixed number of CTAs chosen from its own blob count (about one per 64
+ * blobs), so its arithmetic does not depend on the others. FP32C
  * swimmers the persistent kernel cannot take, and FP64 swimmers, solve on
  * their own with the kernel sequence.
  * The pair products of every instance (M_ss with M_bs, M_sb, ...) run in

@@ -7,9 +7,9 @@
 // step pipelines; the pipelines' kernels overlap on the GPU, so small
 // swimmers that cannot fill the GPU alone fill it together. Work is handed to
 // the workers largest first. The FP32C instances' inner GMRES solves run
-// through a GMRES service (solve.cu): several solves share one cooperative
-// launch of the persistent kernel, each on a fixed number of CTAs chosen from
-// its own size; instances the kernel cannot take, and FP64 instances, use the
+// through a GMRES service (solve.cu): cooperative launches of the persistent
+// kernel run side by side, waiting solves share one, each on a fixed number of
+// CTAs chosen from its own size; instances the kernel cannot take, and FP64 instances, use the
 // kernel-sequence GMRES on their own streams. No instance's arithmetic
 // depends on the others, so each result is the same as when the instance runs
 // alone (a batch of one).

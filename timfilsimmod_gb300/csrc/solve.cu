@@ -342,17 +342,25 @@ int gmres_launch_persistent(tfs_solver *s, const double *rhs, double *f_blobs, d
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Inner solves of several swimmers in one cooperative launch. A swimmer's
-// solve runs on a fixed number of CTAs chosen from its size alone, so its
-// result does not depend on which others share the launch. A waiting thread
-// that finds no launch being prepared becomes the leader: while the previous
-// launch still runs on the GPU (and the waiting solves fill fewer CTAs than
-// the SMs) it lets requests gather, then takes them in arrival order up to
-// the SM count, queues their launch on the service's stream behind each
-// swimmer's inputs, marks each swimmer's completion event and wakes the
-// owners, who wait for that event on their own streams. Launches queue back
-// to back on the service's stream; the host never waits for one to finish
-// except to reuse one of its argument staging slots.
+// Inner solves of several swimmers side by side. A swimmer's solve runs on a
+// fixed number of CTAs chosen from its size alone, so its result does not
+// depend on which others run beside it. A thread that finds no launch being
+// prepared leads: it takes the waiting solves, in arrival order, that fit on
+// the SMs beside the launches in flight (one CTA an SM), queues them as one
+// cooperative launch on a stream of the service behind each swimmer's inputs,
+// and wakes the owners, whose streams wait for its completion. While not even
+// the first fits, or kInFlight launches run already, it lets more gather.
+//
+// The CTAs in flight never exceed the SMs, so all of a launch's CTAs are
+// resident whatever the others do; a full-size launch of a swimmer's own
+// (own_launch) takes its turn among them. With all launches on one stream
+// every solve took as long as the longest beside it, and the next ones waited
+// for that: six swimmers of 16 to 96 filaments on four threads 50 ms a step, 33
+// on streams of their own; twelve of 300 to 640 filaments 164 and 127 ms. A
+// launch for each solve, or as many launches as fit, costs 32 threads more
+// than it gives (64 small swimmers: 148 ms on one stream, 186 and 157); with
+// four in flight 64 swimmers on 16 threads take 190 ms (204 on one stream),
+// on 32 threads 147 to 158, with three 154 to 159.
 // ---------------------------------------------------------------------------
 namespace tfs {
 
@@ -363,89 +371,122 @@ struct GmresService {
     bool done;
     int rc;
   };
-  static constexpr int kSlots = 8;  // host staging of the launch arguments
+  static constexpr int kSlots = 8;
+  static constexpr size_t kInFlight = 4;  // launches at once
   struct Slot {
-    PgArgs *args = nullptr;
-    int2 *map = nullptr;
-    cudaEvent_t copied = nullptr;
+    PgArgs *args = nullptr, *dev_args = nullptr;  // launch arguments, host staging and device
+    int2 *map = nullptr, *dev_map = nullptr;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t copied = nullptr, done = nullptr;
+  };
+  struct Flight {  // a launch that may still run
+    cudaEvent_t done;
+    int ctas;
   };
   std::mutex m;
   std::condition_variable cv;
   std::deque<Req *> pending;
   bool busy = false;
   int sms = 1;
-  cudaStream_t stream = nullptr;
-  PgArgs *dev_args = nullptr;
-  int2 *dev_map = nullptr;
   Slot slot[kSlots];
   int next_slot = 0;
-  cudaEvent_t last = nullptr;  // the latest launch's completion
-  bool launched = false;
+  std::deque<Flight> flights;  // oldest first
   long long launches = 0, solves = 0;
 
-  int waiting_ctas() const {
-    int c = 0;
-    for (const Req *q : pending) c += q->args.P;
-    return c;
+  // CTAs in flight (ended launches leave the list).
+  int in_flight() {
+    int used = 0;
+    for (auto it = flights.begin(); it != flights.end();) {
+      if (cudaEventQuery(it->done) == cudaErrorNotReady) {
+        used += it->ctas;
+        ++it;
+      } else {
+        it = flights.erase(it);
+      }
+    }
+    return used;
   }
-  bool gpu_busy() const { return launched && cudaEventQuery(last) == cudaErrorNotReady; }
 
-  // Queues one launch of the solves in batch (the leader, without the lock).
-  int launch(std::vector<Req *> &batch) {
+  // The next slot; st follows the launch that its event stood for.
+  int take_slot(Slot **out, cudaStream_t st) {
     Slot &sl = slot[next_slot];
     next_slot = (next_slot + 1) % kSlots;
+    if (st == nullptr) st = sl.stream;
+    for (auto it = flights.begin(); it != flights.end();) {
+      if (it->done == sl.done) {
+        TFS_CUDA(cudaStreamWaitEvent(st, sl.done, 0), "service: wait for the slot");
+        it = flights.erase(it);
+      } else {
+        ++it;
+      }
+    }
+    *out = &sl;
+    return TFS_OK;
+  }
+
+  // Queues one launch of the solves in batch (the leader, without the lock;
+  // nobody else touches the slots meanwhile).
+  int launch(std::vector<Req *> &batch, Slot &sl) {
     TFS_CUDA(cudaEventSynchronize(sl.copied), "service: staging slot");
     int ctas = 0;
     size_t dyn = 0;
     for (size_t q = 0; q < batch.size(); ++q) {
       Req *r = batch[q];
-      TFS_CUDA(cudaStreamWaitEvent(stream, r->s->ready_ev, 0), "service: wait for inputs");
-      TFS_CUDA(cudaMemsetAsync(r->args.bar, 0, 4 * sizeof(unsigned), stream), "service: barrier");
+      TFS_CUDA(cudaStreamWaitEvent(sl.stream, r->s->ready_ev, 0), "service: wait for inputs");
+      TFS_CUDA(cudaMemsetAsync(r->args.bar, 0, 4 * sizeof(unsigned), sl.stream),
+               "service: barrier");
       sl.args[q] = r->args;
       for (int c = 0; c < r->args.P; ++c) sl.map[ctas + c] = make_int2((int)q, c);
       ctas += r->args.P;
       dyn = std::max(dyn, r->args.dyn_smem);
     }
-    TFS_CUDA(cudaMemcpyAsync(dev_args, sl.args, sizeof(PgArgs) * batch.size(),
-                             cudaMemcpyHostToDevice, stream),
+    TFS_CUDA(cudaMemcpyAsync(sl.dev_args, sl.args, sizeof(PgArgs) * batch.size(),
+                             cudaMemcpyHostToDevice, sl.stream),
              "service: arguments");
-    TFS_CUDA(cudaMemcpyAsync(dev_map, sl.map, sizeof(int2) * ctas, cudaMemcpyHostToDevice, stream),
+    TFS_CUDA(cudaMemcpyAsync(sl.dev_map, sl.map, sizeof(int2) * ctas, cudaMemcpyHostToDevice,
+                             sl.stream),
              "service: map");
-    TFS_CUDA(cudaEventRecord(sl.copied, stream), "service: staging slot");
-    cudaError_t e = launch_gmres_persistent(dev_args, dev_map, ctas, dyn, 0, stream);
+    TFS_CUDA(cudaEventRecord(sl.copied, sl.stream), "service: staging slot");
+    cudaError_t e = launch_gmres_persistent(sl.dev_args, sl.dev_map, ctas, dyn, 0, sl.stream);
     if (e != cudaSuccess) return cuda_fail(e, "service: persistent GMRES");
-    for (Req *r : batch) TFS_CUDA(cudaEventRecord(r->s->done_ev, stream), "service: completion");
-    TFS_CUDA(cudaEventRecord(last, stream), "service: completion");
+    TFS_CUDA(cudaEventRecord(sl.done, sl.stream), "service: completion");
+    for (Req *r : batch)
+      TFS_CUDA(cudaStreamWaitEvent(r->s->stream, sl.done, 0), "service: wait for the solve");
     return TFS_OK;
   }
 
-  // Queues s's inner solve in a shared launch; s->stream waits for it, and
-  // its scalars (s->gst[0]) are read by the caller's next poll.
+  // Queues s's inner solve; s->stream waits for it, and its scalars
+  // (s->gst[0]) are read by the caller's next poll.
   int solve(tfs_solver *s, const double *rhs, double *f_blobs, double *v_bodies, double tol) {
     Req r{s, persistent_args(s, s->pg_group, rhs, f_blobs, v_bodies, tol, 0), false, TFS_OK};
     TFS_CUDA(cudaEventRecord(s->ready_ev, s->stream), "service: inputs ready");
     std::unique_lock<std::mutex> g(m);
     pending.push_back(&r);
-    cv.notify_all();
     while (!r.done) {
       if (busy) {
         cv.wait(g);
         continue;
       }
       busy = true;
-      while (waiting_ctas() < sms && gpu_busy()) cv.wait_for(g, std::chrono::microseconds(20));
+      int used;
+      while ((used = in_flight()) > 0 &&
+             (flights.size() >= kInFlight || used + pending.front()->args.P > sms))
+        cv.wait_for(g, std::chrono::microseconds(20));
       std::vector<Req *> batch;
       int ctas = 0;
-      while (!pending.empty() && (batch.empty() || ctas + pending.front()->args.P <= sms)) {
+      while (!pending.empty() &&
+             (batch.empty() || used + ctas + pending.front()->args.P <= sms)) {
         ctas += pending.front()->args.P;
         batch.push_back(pending.front());
         pending.pop_front();
       }
+      Slot *sl = nullptr;
+      int lrc = take_slot(&sl, nullptr);
       g.unlock();
-      const int lrc = launch(batch);
+      if (lrc == TFS_OK) lrc = launch(batch, *sl);
       g.lock();
       if (lrc == TFS_OK) {
-        launched = true;
+        flights.push_back({sl->done, ctas});
         ++launches;
         solves += (long long)batch.size();
       }
@@ -456,9 +497,24 @@ struct GmresService {
       busy = false;
       cv.notify_all();
     }
-    g.unlock();
-    if (r.rc != TFS_OK) return r.rc;
-    TFS_CUDA(cudaStreamWaitEvent(s->stream, s->done_ev, 0), "service: wait for the solve");
+    return r.rc;
+  }
+
+  // A launch of s's own on all SMs, on s->stream: after the launches in
+  // flight, before those that follow.
+  template <typename F>
+  int own_launch(tfs_solver *s, F launch_it) {
+    std::unique_lock<std::mutex> g(m);
+    cv.wait(g, [&] { return !busy; });
+    Slot *sl = nullptr;
+    int rc = take_slot(&sl, s->stream);
+    if (rc != TFS_OK) return rc;
+    for (const Flight &f : flights)
+      TFS_CUDA(cudaStreamWaitEvent(s->stream, f.done, 0), "service: wait for CTAs");
+    flights.clear();
+    if ((rc = launch_it()) != TFS_OK) return rc;
+    TFS_CUDA(cudaEventRecord(sl->done, s->stream), "service: completion");
+    flights.push_back({sl->done, sms});
     return TFS_OK;
   }
 };
@@ -467,14 +523,15 @@ GmresService *service_create() {
   GmresService *sv = new (std::nothrow) GmresService();
   if (sv == nullptr) return nullptr;
   sv->sms = num_sms();
-  bool ok = cudaStreamCreateWithFlags(&sv->stream, cudaStreamNonBlocking) == cudaSuccess &&
-            cudaMalloc(&sv->dev_args, sizeof(PgArgs) * kMaxPgCtas) == cudaSuccess &&
-            cudaMalloc(&sv->dev_map, sizeof(int2) * kMaxPgCtas) == cudaSuccess &&
-            cudaEventCreateWithFlags(&sv->last, cudaEventDisableTiming) == cudaSuccess;
+  bool ok = true;
   for (auto &sl : sv->slot)
-    ok = ok && cudaHostAlloc(&sl.args, sizeof(PgArgs) * kMaxPgCtas, cudaHostAllocDefault) == cudaSuccess &&
+    ok = ok && cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking) == cudaSuccess &&
+         cudaMalloc(&sl.dev_args, sizeof(PgArgs) * kMaxPgCtas) == cudaSuccess &&
+         cudaMalloc(&sl.dev_map, sizeof(int2) * kMaxPgCtas) == cudaSuccess &&
+         cudaHostAlloc(&sl.args, sizeof(PgArgs) * kMaxPgCtas, cudaHostAllocDefault) == cudaSuccess &&
          cudaHostAlloc(&sl.map, sizeof(int2) * kMaxPgCtas, cudaHostAllocDefault) == cudaSuccess &&
-         cudaEventCreateWithFlags(&sl.copied, cudaEventDisableTiming) == cudaSuccess;
+         cudaEventCreateWithFlags(&sl.copied, cudaEventDisableTiming) == cudaSuccess &&
+         cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     service_destroy(sv);
@@ -485,16 +542,16 @@ GmresService *service_create() {
 
 void service_destroy(GmresService *sv) {
   if (sv == nullptr) return;
-  if (sv->stream) cudaStreamSynchronize(sv->stream);
-  if (sv->dev_args) cudaFree(sv->dev_args);
-  if (sv->dev_map) cudaFree(sv->dev_map);
   for (auto &sl : sv->slot) {
+    if (sl.stream) cudaStreamSynchronize(sl.stream);
+    if (sl.dev_args) cudaFree(sl.dev_args);
+    if (sl.dev_map) cudaFree(sl.dev_map);
     if (sl.args) cudaFreeHost(sl.args);
     if (sl.map) cudaFreeHost(sl.map);
     if (sl.copied) cudaEventDestroy(sl.copied);
+    if (sl.done) cudaEventDestroy(sl.done);
+    if (sl.stream) cudaStreamDestroy(sl.stream);
   }
-  if (sv->last) cudaEventDestroy(sv->last);
-  if (sv->stream) cudaStreamDestroy(sv->stream);
   delete sv;
 }
 
@@ -510,11 +567,11 @@ int service_attach(GmresService *sv, tfs_solver *s) {
   PgShape sh{};
   if (!pg_grid(nb, want, s->max_iter, &sh) || sh.G > s->pg.G || sh.S > s->pg.S)
     return fail(TFS_ESTATE, "no persistent GMRES shape for %d blobs on %d CTAs", nb, want);
-  for (cudaEvent_t *ev : {&s->ready_ev, &s->done_ev})
-    if (*ev == nullptr && cudaEventCreateWithFlags(ev, cudaEventDisableTiming) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(TFS_ECUDA, "event creation failed");
-    }
+  if (s->ready_ev == nullptr &&
+      cudaEventCreateWithFlags(&s->ready_ev, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(TFS_ECUDA, "event creation failed");
+  }
   s->pg_group = sh;
   s->service = sv;
   return TFS_OK;
@@ -594,7 +651,10 @@ int refine_cycles(tfs_solver *s, const GmresArgs &g64, int vec64, bool first_rea
       if ((rc = s->service->solve(s, s->r, s->dx, s->dx + vel, itol)) != TFS_OK) return rc;
       pending = true;
     } else if (own) {
-      if ((rc = gmres_launch_persistent(s, s->r, s->dx, s->dx + vel, itol, vec64)) != TFS_OK)
+      auto launch_it = [&] {
+        return gmres_launch_persistent(s, s->r, s->dx, s->dx + vel, itol, vec64);
+      };
+      if ((rc = s->service ? s->service->own_launch(s, launch_it) : launch_it()) != TFS_OK)
         return rc;
       pending = true;
     } else {
@@ -818,8 +878,7 @@ void solve_free(tfs_solver *s) {
   s->aux_stream = nullptr;
   s->aux_fork = s->aux_join = nullptr;
   if (s->ready_ev) cudaEventDestroy(s->ready_ev);
-  if (s->done_ev) cudaEventDestroy(s->done_ev);
-  s->ready_ev = s->done_ev = nullptr;
+  s->ready_ev = nullptr;
   for (auto &g : s->chunk_graphs) cudaGraphExecDestroy(g.exec);
   s->chunk_graphs.clear();
   double *bufs[] = {s->refs, s->diff, s->mats, s->Q, s->H, s->beta, s->cs, s->sn, s->y, s->z,

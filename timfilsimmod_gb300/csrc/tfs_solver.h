@@ -96,12 +96,11 @@ struct tfs_solver {
   unsigned *pg_bar = nullptr;
   tfs::PgArgs *pg_gp = nullptr;  // device copy of this solve's arguments
   int2 *pg_cmap = nullptr;       // CTA c -> (0, c)
-  // inner solves shared with other swimmers' (one cooperative launch for all
-  // that are waiting): the service, this swimmer's fixed shape within such a
-  // launch, and events marking its inputs ready and its solve ended
+  // inner solves beside other swimmers': the service, this swimmer's fixed
+  // shape within a shared launch, and an event marking its inputs ready
   tfs::GmresService *service = nullptr;
   tfs::PgShape pg_group{};
-  cudaEvent_t ready_ev = nullptr, done_ev = nullptr;
+  cudaEvent_t ready_ev = nullptr;
   tfs::GmresScalars *gst_host = nullptr;  // pinned copies
   double *f6_host = nullptr;              // pinned 6
   int last_iters = 0, last_outer = 0;

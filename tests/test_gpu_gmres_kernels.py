@@ -1,11 +1,11 @@
-"""The Arnoldi kernels of the free-body GMRES (csrc/gmres.cu) against a dense
-FP64 solve, at slices of one blob and of many, and at Krylov spaces below and
+"""The Arnoldi kernels of the free-body GMRES (csrc/gmres.cu; FP32C: the
+cooperative kernel of csrc/gmres_persistent.cu) against a dense FP64 solve, at slices of one blob and of many, and at Krylov spaces below and
 above one group (16) and one pass (64) of columns.
 
 Tolerances: the solve stops at 1e-10 of ||rhs||. Blob forces within 1e-8 (spaced
 blobs: condition of order 10), the bar of the other FP64 solves; overlapping
 ones are ill-conditioned, so there it is the residual that is checked, within
-1e-8. 27 000 blobs (slices longer than the rows kept in shared memory): the
+1e-8 (FP32C, refined to 1e-8: 2e-8). 27 000 blobs (slices longer than the rows kept in shared memory): the
 residual that three columns leave is the estimate, within 1e-6."""
 import numpy as np
 import pytest
@@ -38,10 +38,10 @@ def dense(refs):
     return np.block([[M.reshape(3 * nb, 3 * nb) / (8 * np.pi), -K], [-K.T, np.zeros((6, 6))]])
 
 
-def solver(refs, tol, cols):
+def solver(refs, tol, cols, precision="fp64"):
     from timfilsimmod_gb300.mobility import RpyMobilitySolver
 
-    s = RpyMobilitySolver(1, 2, 12, len(refs), precision="fp64")
+    s = RpyMobilitySolver(1, 2, 12, len(refs), precision=precision)
     s.set_blob_references(refs)
     s.set_body_pose([0.1, -0.3, 0.7], [1.0, 0.0, 0.0, 0.0])
     s.set_linear_solver(tol, cols)
@@ -69,6 +69,19 @@ def test_many_columns(gap):
     s.finalise()
     assert iters > 16
     assert np.linalg.norm(rhs - dense(refs) @ x) <= 1e-8 * np.linalg.norm(rhs)
+
+
+@pytest.mark.parametrize("nb,gap", [(3, 3.0), (65, 1.5), (257, 2.0), (642, 1.0), (642, 0.8)])
+def test_cooperative_kernel(nb, gap):
+    refs = sphere(nb, gap * max(1.0, (nb / 12.0) ** 0.5))
+    rhs = np.random.default_rng(nb).normal(size=3 * nb + 6)
+    s = solver(refs, 1e-8, min(350, 3 * nb + 6), "fp32c")
+    s.set_persistent_gmres(True)
+    s.set_refinement_vectors("fp64")  # FP32 vectors can't take these body rows
+    s.solve_linear_system(rhs)
+    x = np.concatenate([s.blob_forces().ravel(), s.body_velocities().ravel()])
+    s.finalise()
+    assert np.linalg.norm(rhs - dense(refs) @ x) <= 2e-8 * np.linalg.norm(rhs)
 
 
 def test_long_slices():

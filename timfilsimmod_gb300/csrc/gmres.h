@@ -71,7 +71,7 @@ struct PgArgs {
   float2 *mpart;          // S * 3 nb: split partial products of M_bb, (hi, lo)
   // per-CTA partials, FP64-sized buffers holding values of the vector type:
   double *p6, *ps;        // partial 6-vectors and sums of squares
-  double *pd1, *pd2;      // Gram-Schmidt partial dots ((max_iter + 2) * G each)
+  double *pd1, *pd2;      // Gram-Schmidt partial sums and dots ((8 + max_iter + 2) * G each)
   double *aux;            // control words (3), then h1, h2, y (vector type) published by CTAs
   unsigned *bar;          // 4: barrier count, generation, abort
   int P, TB, tbs, S, chunk, Kr;  // P: the CTAs of this solve
@@ -90,9 +90,9 @@ struct PgArgs {
 // (no occupancy, or more than kMaxPgBlobsPerCta blobs per CTA).
 int pg_grid(int nb, int sms, int max_iter, PgShape *shape);
 // Buffer sizes (elements) of one shape.
-inline size_t pg_p6_elems(const PgShape &s) { return 6 * 6 * (size_t)s.G; }
-inline size_t pg_ps_elems(const PgShape &s) { return 3 * (size_t)s.G; }
-inline size_t pg_pd_elems(const PgShape &s) { return 352 * (size_t)s.G; }
+inline size_t pg_p6_elems(const PgShape &s) { return 5 * 6 * (size_t)s.G; }
+inline size_t pg_ps_elems(const PgShape &s) { return 2 * (size_t)s.G; }
+inline size_t pg_pd_elems(const PgShape &s) { return (8 + 352) * (size_t)s.G + 2; }
 constexpr size_t kPgAuxElems = 3 + 3 * 352;
 // One cooperative launch of `ctas` CTAs running the solves in gp[] (device
 // array): CTA c works for solve cmap[c].x as its CTA cmap[c].y. Every solve's

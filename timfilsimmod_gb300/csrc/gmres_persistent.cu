@@ -42,6 +42,17 @@
 // each row's owner adds the splits in order. One launch may carry several
 // independent solves (PgArgs array + CTA map), each on its own CTAs.
 //
+// What bounds an Arnoldi step: not arithmetic but a chain of some thirty short
+// phases, each run once a step with its instructions to be fetched anew. So the
+// loops outside M_bb are not unrolled (the same code unrolled by the compiler's
+// default: 10% slower), independent sums run on other warps, and the M_bb
+// targets stay on the SM. 24.9 -> 21.6 us a step at 2 562 blobs (M_bb with its
+// barrier 10.3 -> 9.3, the last phase 3.5 -> 1.2), bit for bit the same. Tried
+// and left out, as they change rounding, which an implicit step's body
+// displacement amplifies to 1e-4: two sources a packed instruction in M_bb (8.9
+// us), and one Gram-Schmidt pass corrected by the basis' Gram matrix (20.3 us a
+// step in all).
+//
 // Grid barrier: one monotonic arrival counter per solve in global memory
 // (the e-th barrier passes at e x P arrivals). Every wait is bounded (2 s of
 // globaltimer, plus an iteration cap); a CTA that gives up raises an abort
@@ -54,7 +65,7 @@
 #include <algorithm>
 
 #include "gmres.h"
-#include "rpy_tile.cuh"
+#include "rpy_pair2.cuh"
 #include "tfs_kernels.h"
 
 namespace tfs {
@@ -67,6 +78,9 @@ constexpr int kPTS = 128;      // sources per shared-memory tile of M_bb
 constexpr int kPK = 352;       // Krylov columns + 1 (max_iter <= 350)
 constexpr int kMaxRows = 3 * kMaxPgBlobsPerCta;
 constexpr int kHB = 4096;      // doubles of the staging buffer (H columns, M_bb partials)
+// A slice's rows times splits up to which a row's splits are added by several
+// threads (beyond: by one, staged)
+constexpr int kSplitsAtOnce = 4096;
 
 // bytes of dynamic shared memory before the resident Krylov rows (vectors of V)
 template <typename V>
@@ -77,10 +91,18 @@ constexpr size_t pg_dyn_fixed() {
 // control words CTA 0 publishes each Arnoldi step
 enum { C_FINISH = 0, C_REL, C_STATUS, kCtl };
 
-// p6 slots: per-CTA partial 6-vectors sum_m (l_m ; d_m x l_m)
-enum { K_SOLN = 0, K_R0, K_RHS, K_Z, K_W, K_T, kP6Slots };
+// p6 slots: per-CTA partial 6-vectors sum_m (l_m ; d_m x l_m); K_Z, staged by
+// 16-byte loads, starts the buffer
+enum { K_Z = 0, K_SOLN, K_R0, K_RHS, K_T, kP6Slots };
 // ps slots: per-CTA partial sums of squares
-enum { S_RHS = 0, S_R0, S_NORM, kPsSlots };
+enum { S_RHS = 0, S_R0, kPsSlots };
+
+// Rows of a Gram-Schmidt pass' partials (pd1, pd2), G of them a row, staged with
+// one sweep: the sum of squares and the body sums of w (second pass; a row of
+// no meaning after them keeps the dots on a 16-byte boundary), then the dots of
+// each column.
+constexpr int kSums = 8;
+
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -262,60 +284,66 @@ __device__ void cta_sums(const V *buf, int G, int count, V *out, V *cst) {
   __syncthreads();
 }
 
-// This CTA's partials of the slice rows ls: warp j < 6 sums component j of
-// sum_m (l_m ; d_m x l_m) into p6 slot kt_slot and, with sq_slot >= 0, warp
-// 6 the sum of squares into ps slot sq_slot (lanes stride over blobs or
-// rows, then a fixed shuffle tree). No barrier; ls must be complete.
+// This CTA's partials of the slice rows ls: the last warp but j < 6 sums
+// component j of sum_m (l_m ; d_m x l_m) into row j of kt and, with sq, the
+// next one the sum of squares into sq (lanes stride over blobs or rows, then
+// a fixed shuffle tree): the last warps, as the first ones have the dots of
+// few columns to do. No barrier; ls must be
+// complete.
 template <typename V>
-__device__ void slice_partials(const PgArgs &p, const PSlice<V> &sl, const V *ls, int kt_slot,
-                               int sq_slot) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (!sl.owner || wid >= (sq_slot >= 0 ? 7 : 6)) return;
+__device__ void slice_partials(const PgArgs &p, const PSlice<V> &sl, const V *ls, V *kt, V *sq) {
+  const int lane = threadIdx.x & 31, wid = kPW - 1 - (int)(threadIdx.x >> 5);
+  if (!sl.owner || wid >= (sq ? 7 : 6)) return;
   V s = V(0);
   if (wid < 3) {
+#pragma unroll 1
     for (int m = sl.m0 + lane; m < sl.m1; m += 32) s += ls[3 * (m - sl.m0) + wid];
   } else if (wid < 6) {  // (d x l)_j = d_a l_b - d_b l_a, (a, b) = (j + 1, j + 2) mod 3
     const int a = (wid - 2) % 3, b = (wid - 1) % 3;
+#pragma unroll 1
     for (int m = sl.m0 + lane; m < sl.m1; m += 32) {
       const V *d = sl.d + 3 * (m - sl.m0);
       const V *v = ls + 3 * (m - sl.m0);
       s += d[a] * v[b] - d[b] * v[a];
     }
   } else {
+#pragma unroll 1
     for (int r = lane; r < sl.rows; r += 32) s += ls[r] * ls[r];
   }
   s = warp_sum(s);
-  if (lane == 0) {
-    const int G = p.g.G, c = p.rank;
-    if (wid < 6) reinterpret_cast<V *>(p.p6)[(size_t)(kt_slot * 6 + wid) * G + c] = s;
-    else reinterpret_cast<V *>(p.ps)[(size_t)sq_slot * G + c] = s;
-  }
+  if (lane == 0) (wid < 6 ? kt + (size_t)wid * p.g.G : sq)[p.rank] = s;
 }
 
 // z = P^-1 (q rows of the slice in shared memory, q_vel), given
 // bsum = sum_m (q_m ; d_m x q_m) / bscale: b = -bsum * bscale, the body part
 // (U', Omega') = KTKinv b - N q_vel (mobility_solver.cpp:1437-1509), then
 // z_m = 6 pi mu a (q_m + U' + Omega' x d_m). Writes zv (6, shared) and the
-// slice's z rows into zs (shared); ends with a barrier.
+// slice's z rows into zs (shared); ends with a barrier. precond_body: the body
+// part, by one warp; precond_rows: the rows; no barriers.
 template <typename V>
-__device__ void precond(const PgArgs &p, const PSlice<V> &sl, const V *qs, const V *qvel,
-                        const V *bsum, V bscale, V *zs, V *zv, const V *mats) {
-  if (threadIdx.x < 6) {
-    const int i = threadIdx.x;
-    const V *N = mats, *Kinv = mats + 36;
-    V t1 = V(0), t2 = V(0);
-    V u1 = V(0), u2 = V(0);
-    for (int k = 0; k < 6; k += 2) {
-      t1 += Kinv[i + 6 * k] * (-bsum[k] * bscale);
-      u1 += Kinv[i + 6 * (k + 1)] * (-bsum[k + 1] * bscale);
-      t2 += N[i + 6 * k] * qvel[k];
-      u2 += N[i + 6 * (k + 1)] * qvel[k + 1];
-    }
-    zv[i] = (t1 + u1) - (t2 + u2);
+__device__ __forceinline__ void precond_body(const V *qvel, const V *bsum, V bscale, V *zv,
+                                             const V *mats) {
+  const int i = threadIdx.x & 31;
+  if (i >= 6) return;
+  const V *N = mats, *Kinv = mats + 36;
+  V t1 = V(0), t2 = V(0);
+  V u1 = V(0), u2 = V(0);
+#pragma unroll
+  for (int k = 0; k < 6; k += 2) {
+    t1 += Kinv[i + 6 * k] * (-bsum[k] * bscale);
+    u1 += Kinv[i + 6 * (k + 1)] * (-bsum[k + 1] * bscale);
+    t2 += N[i + 6 * k] * qvel[k];
+    u2 += N[i + 6 * (k + 1)] * qvel[k + 1];
   }
-  __syncthreads();
+  zv[i] = (t1 + u1) - (t2 + u2);
+}
+
+template <typename V>
+__device__ __forceinline__ void precond_rows(const PgArgs &p, const PSlice<V> &sl, const V *qs,
+                                             V *zs, const V *zv) {
   const V u0 = zv[0], u1 = zv[1], u2 = zv[2], w0 = zv[3], w1 = zv[4], w2 = zv[5];
   const V minv = V(p.minv);
+#pragma unroll 1
   for (int m = sl.m0 + threadIdx.x; m < sl.m1; m += kPB) {
     const V *d = sl.d + 3 * (m - sl.m0);
     const V *l = qs + 3 * (m - sl.m0);
@@ -328,12 +356,21 @@ __device__ void precond(const PgArgs &p, const PSlice<V> &sl, const V *qs, const
     o[1] = minv * b1;
     o[2] = minv * b2;
   }
+}
+
+template <typename V>
+__device__ void precond(const PgArgs &p, const PSlice<V> &sl, const V *qs, const V *qvel,
+                        const V *bsum, V bscale, V *zs, V *zv, const V *mats) {
+  if (threadIdx.x < 32) precond_body(qvel, bsum, bscale, zv, mats);
+  __syncthreads();
+  precond_rows(p, sl, qs, zs, zv);
   __syncthreads();
 }
 
 // FP32 source records {x - origin, f, 0, 0} of the slice's blobs for M_bb.
 template <typename V>
 __device__ void pack_records(const PgArgs &p, const PSlice<V> &sl, const V *fs) {
+#pragma unroll 1
   for (int m = sl.m0 + threadIdx.x; m < sl.m1; m += kPB) {
     const V *f = fs + 3 * (m - sl.m0);
     float4 a, b;
@@ -351,37 +388,79 @@ __device__ void pack_records(const PgArgs &p, const PSlice<V> &sl, const V *fs) 
   }
 }
 
-// One staged tile of M_bb for the NT targets of this thread (NT = 1 in a
-// warp where no lane has a second target), FP32 pairs; the tile's sum is
+// The pairs of one staged tile inside the contact distance of a target, by the
+// full formula, added to its sum.
+__device__ __forceinline__ float3 mbb_near(float3 w, float x, float y, float z, const float *src,
+                                        int cnt, float a, float asum2) {
+  PairConst<float> pc;
+  pc.ai = pc.aj = a;
+  pc.asum2 = asum2;
+  pc.s = pc.s3 = 0.f;  // the far field's
+  const float xt[1] = {x}, yt[1] = {y}, zt[1] = {z};
+  const unsigned nf[1] = {1u};
+  float v[1][3] = {{w.x, w.y, w.z}};
+  near_pass<float, 3, 3, 1>(v, xt, yt, zt, nf, src, cnt, pc);
+  return make_float3(v[0][0], v[0][1], v[0][2]);
+}
+
+// One staged tile of M_bb for the targets of this thread, FP32 pairs: both
+// (TWO) in the halves of packed FP32x2 instructions, or the first alone in a
+// warp where no lane has a second. Each half rounds as the plain instruction
+// does, so a target's sum does not depend on its company. The tile's sum is
 // added compensated into (hi, lo).
-template <int NT>
+template <bool TWO>
 __device__ __forceinline__ void mbb_tile(const float (&xt)[2], const float (&yt)[2],
                                          const float (&zt)[2], const int (&i)[2], int base,
                                          int cnt, const float *src, const PairConst<float> &pc,
                                          float (&hi)[2][3], float (&lo)[2][3]) {
-  float x[NT], y[NT], z[NT], v[NT][3];
+  constexpr int NT = TWO ? 2 : 1;
+  float v[NT][3];
   unsigned nf[NT];  // pairs inside the contact distance
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
-    x[t] = xt[t];
-    y[t] = yt[t];
-    z[t] = zt[t];
     nf[t] = 0u;
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[t][k] = 0.f;
   }
+  if constexpr (TWO) {
+    const float2 x = make_float2(xt[0], xt[1]), y = make_float2(yt[0], yt[1]),
+                 z = make_float2(zt[0], zt[1]), s = both(pc.s), s3 = both(pc.s3);
+    float2 w[3] = {both(0.f), both(0.f), both(0.f)};
 #pragma unroll 2
-  for (int j = 0; j < cnt; ++j) {
-    float sx, sy, sz, f[3];
-    RecLoad<float, 3>::get(src + 8 * j, sx, sy, sz, f);
+    for (int j = 0; j < cnt; ++j) {
+      float sx, sy, sz, f[3];
+      RecLoad<float, 3>::get(src + 8 * j, sx, sy, sz, f);
+      const float2 dx = add2(x, both(-sx)), dy = add2(y, both(-sy)), dz = add2(z, both(-sz));
+      const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+      const bool f0 = r2.x > pc.asum2, f1 = r2.y > pc.asum2;
+      nf[0] += f0 ? 0u : 1u;
+      nf[1] += f1 ? 0u : 1u;
+      const float2 rm1 =
+          make_float2(f0 ? rsqrt_ftz(r2.x) : 0.f, f1 ? rsqrt_ftz(r2.y) : 0.f);
+      // far_pair<float, 3, 3>, operation by operation
+      const float2 rm2 = mul2(rm1, rm1), rm3 = mul2(rm1, rm2), rm5 = mul2(rm3, rm2);
+      const float2 A = fma2(s, rm3, rm1), B = fma2(s3, rm5, rm3);
+      const float2 dF = fma2(dx, both(f[0]), fma2(dy, both(f[1]), mul2(dz, both(f[2]))));
+      const float2 Bd = mul2(B, dF);
+      w[0] = fma2(A, both(f[0]), fma2(Bd, dx, w[0]));
+      w[1] = fma2(A, both(f[1]), fma2(Bd, dy, w[1]));
+      w[2] = fma2(A, both(f[2]), fma2(Bd, dz, w[2]));
+    }
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      const float dx = x[t] - sx, dy = y[t] - sy, dz = z[t] - sz;
+    for (int k = 0; k < 3; ++k) {
+      v[0][k] = w[k].x;
+      v[NT - 1][k] = w[k].y;
+    }
+  } else {
+#pragma unroll 2
+    for (int j = 0; j < cnt; ++j) {
+      float sx, sy, sz, f[3];
+      RecLoad<float, 3>::get(src + 8 * j, sx, sy, sz, f);
+      const float dx = xt[0] - sx, dy = yt[0] - sy, dz = zt[0] - sz;
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
       const bool far = r2 > pc.asum2;
-      nf[t] += far ? 0u : 1u;
-      const float rs = rsqrt_far(r2);
-      far_pair<float, 3, 3>(v[t], dx, dy, dz, far ? rs : 0.f, f, pc);
+      nf[0] += far ? 0u : 1u;
+      far_pair<float, 3, 3>(v[0], dx, dy, dz, far ? rsqrt_ftz(r2) : 0.f, f, pc);
     }
   }
   // a target whose only pair inside the contact distance in this tile is
@@ -398,19 +477,18 @@ __device__ __forceinline__ void mbb_tile(const float (&xt)[2], const float (&yt)
         RecLoad<float, 3>::get(src + 8 * js, sx, sy, sz, f);
         const float A = 4.f / (3.f * pc.ai);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) v[t][k] += A * f[k];
+        for (int k = 0; k < 3; ++k) v[t][k] = fmaf(A, f[k], v[t][k]);
       }
-      nf[t] = 0u;
+    } else {
+      const float3 w = mbb_near(make_float3(v[t][0], v[t][1], v[t][2]), xt[t], yt[t], zt[t], src,
+                                cnt, pc.ai, pc.asum2);
+      v[t][0] = w.x;
+      v[t][1] = w.y;
+      v[t][2] = w.z;
     }
-  }
-  unsigned any = 0u;
-#pragma unroll
-  for (int t = 0; t < NT; ++t) any |= nf[t];
-  if (__any_sync(0xffffffffu, any != 0u)) near_pass<float, 3, 3, NT>(v, x, y, z, nf, src, cnt, pc);
-#pragma unroll
-  for (int t = 0; t < NT; ++t)
 #pragma unroll
     for (int k = 0; k < 3; ++k) two_sum(hi[t][k], lo[t][k], v[t][k]);
+  }
 }
 
 // M_bb of the packed records: (target block x source split) units over the
@@ -419,7 +497,11 @@ __device__ __forceinline__ void mbb_tile(const float (&xt)[2], const float (&yt)
 // pass), FP32 pairs, per-tile compensated sums; each split's sum is written
 // as its (hi, lo) FP32 pair mpart[(split * nb + target) * 3 + k] (the
 // consumer adds the splits compensated and scales by 1 / (8 pi mu)).
-__device__ void mbb_units(const PgArgs &p, float *src) {
+//
+// A CTA has one unit where they are no more than the CTAs: its targets' positions
+// stay in shared memory (tx, of unit held) from one product to the next.
+__device__ __forceinline__ void mbb_units(const PgArgs &p, float *src, float (*tx)[kPB],
+                                          int &held) {
   const int nb = p.g.nb;
   const int units = p.TB * p.S;
   const int first = p.P > 1 ? 1 : 0, workers = p.P - first;
@@ -430,6 +512,7 @@ __device__ void mbb_units(const PgArgs &p, float *src) {
   pc.asum2 = p.pc_asum2;
   pc.s = p.pc_s;
   pc.s3 = p.pc_s3;
+#pragma unroll 1
   for (int u = p.rank - first; u < units; u += workers) {
     const int tb = u / p.S, sp = u - tb * p.S;
     const int t0 = tb * p.tbs, t1 = min(nb, t0 + p.tbs);
@@ -443,24 +526,32 @@ __device__ void mbb_units(const PgArgs &p, float *src) {
       i[t] = t0 + (int)threadIdx.x + t * kPB;
       act[t] = i[t] < t1;
       if (!act[t]) i[t] = t1 - 1;
-      xt[t] = __ldcg(p.x32 + 3 * (size_t)i[t]);
-      yt[t] = __ldcg(p.x32 + 3 * (size_t)i[t] + 1);
-      zt[t] = __ldcg(p.x32 + 3 * (size_t)i[t] + 2);
+      if (held != u) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          tx[3 * t + k][threadIdx.x] = __ldcg(p.x32 + 3 * (size_t)i[t] + k);
+      }
+      xt[t] = tx[3 * t][threadIdx.x];
+      yt[t] = tx[3 * t + 1][threadIdx.x];
+      zt[t] = tx[3 * t + 2][threadIdx.x];
 #pragma unroll
       for (int k = 0; k < 3; ++k) hi[t][k] = lo[t][k] = 0.f;
     }
+    held = u;
     const bool warp_active = __any_sync(0xffffffffu, act[0] || act[1]);
     const bool two = __any_sync(0xffffffffu, act[1]);
+#pragma unroll 1
     for (int base = s0; base < s1; base += kPTS) {
       const int cnt = min(kPTS, s1 - base);
       __syncthreads();
       const float4 *g = reinterpret_cast<const float4 *>(p.rec + 8 * (size_t)base);
       float4 *d = reinterpret_cast<float4 *>(src);
+#pragma unroll 1
       for (int q = threadIdx.x; q < 2 * cnt; q += kPB) d[q] = __ldcg(g + q);
       __syncthreads();
       if (!warp_active) continue;
-      if (two) mbb_tile<2>(xt, yt, zt, i, base, cnt, src, pc, hi, lo);
-      else mbb_tile<1>(xt, yt, zt, i, base, cnt, src, pc, hi, lo);
+      if (two) mbb_tile<true>(xt, yt, zt, i, base, cnt, src, pc, hi, lo);
+      else mbb_tile<false>(xt, yt, zt, i, base, cnt, src, pc, hi, lo);
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
@@ -482,17 +573,22 @@ __device__ void apply_rows(const PgArgs &p, const PSlice<V> &sl, const V *zv, V 
   const int nb = p.g.nb, rows = sl.rows;
   const int per = rows > 0 ? max(1, kHB / rows) : 1;  // splits per staging round
   float2 *st2 = reinterpret_cast<float2 *>(stage);
+#pragma unroll 1
   for (int r = threadIdx.x; r < rows; r += kPB) acc[r] = make_float2(0.f, 0.f);
+#pragma unroll 1
   for (int s0 = 0; s0 < p.S; s0 += per) {
     const int s1 = min(p.S, s0 + per);
     __syncthreads();
+#pragma unroll 1
     for (int q = threadIdx.x; q < (s1 - s0) * rows; q += kPB) {
       const int s = s0 + q / rows, r = q - (q / rows) * rows;
       st2[q] = __ldcg(p.mpart + ((size_t)s * nb + sl.m0) * 3 + r);
     }
     __syncthreads();
+#pragma unroll 1
     for (int r = threadIdx.x; r < rows; r += kPB) {
       float h = acc[r].x, l = acc[r].y;
+#pragma unroll 1
       for (int s = 0; s < s1 - s0; ++s) {
         two_sum(h, l, st2[s * rows + r].x);
         l += st2[s * rows + r].y;
@@ -502,6 +598,7 @@ __device__ void apply_rows(const PgArgs &p, const PSlice<V> &sl, const V *zv, V 
   }
   __syncthreads();
   const V scale = V(p.scale);
+#pragma unroll 1
   for (int r = threadIdx.x; r < rows; r += kPB) {
     const int m = sl.m0 + r / 3, j = r - 3 * (r / 3);
     const V *d = sl.d + 3 * (m - sl.m0);
@@ -534,6 +631,7 @@ __device__ __forceinline__ V qrow(const PgArgs &p, const PSlice<V> &sl, const V 
 // memory beyond the resident columns).
 template <typename V>
 __device__ void store_q(const PgArgs &p, const PSlice<V> &sl, V *qres, int i, const V *ws) {
+#pragma unroll 1
   for (int r = threadIdx.x; r < sl.rows; r += kPB) {
     if (i < p.Kr) qres[(size_t)i * sl.rows + r] = ws[r];
     else qglobal<V>(p)[(size_t)i * p.g.n + 3 * (size_t)sl.m0 + r] = ws[r];
@@ -549,6 +647,7 @@ __device__ void slice_dots(const PgArgs &p, const PSlice<V> &sl, const V *ws, in
   if (!sl.owner) return;
   const int tpi = k <= kPB / 16 ? 16 : k <= kPB / 8 ? 8 : 4;
   const int part = threadIdx.x & (tpi - 1);
+#pragma unroll 1
   for (int i0 = 0; i0 < k; i0 += kPB / tpi) {
     const int i = i0 + (int)threadIdx.x / tpi;
     V s = V(0), u = V(0);
@@ -556,16 +655,19 @@ __device__ void slice_dots(const PgArgs &p, const PSlice<V> &sl, const V *ws, in
       int r = part;
       if (i < p.Kr) {
         const V *q = qres + (size_t)i * sl.rows;
+#pragma unroll 1
         for (; r + tpi < sl.rows; r += 2 * tpi) {
           s += ws[r] * q[r];
           u += ws[r + tpi] * q[r + tpi];
         }
         if (r < sl.rows) s += ws[r] * q[r];
       } else {
+#pragma unroll 1
         for (; r < sl.rows; r += tpi) s += ws[r] * qrow(p, sl, qres, i, r);
       }
     }
     s += u;
+#pragma unroll 1
     for (int o = 1; o < tpi; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (i < k && part == 0) pd[(size_t)i * p.g.G + p.rank] = s;
   }
@@ -582,6 +684,7 @@ __device__ void slice_axpy(const PgArgs &p, const PSlice<V> &sl, const V *h, int
     V t = V(0), u = V(0);
     if (r < sl.rows) {
       int i = sub;
+#pragma unroll 1
       for (; i + 4 < k; i += 8) {
         t += h[i] * qrow(p, sl, qres, i, r);
         u += h[i + 4] * qrow(p, sl, qres, i + 4, r);
@@ -593,12 +696,15 @@ __device__ void slice_axpy(const PgArgs &p, const PSlice<V> &sl, const V *h, int
     t += __shfl_xor_sync(0xffffffffu, t, 2);
     if (r < sl.rows && sub == 0) ws[r] += sign * t;
   } else {
+#pragma unroll 1
     for (int r = threadIdx.x; r < sl.rows; r += kPB) {
       V t[4] = {V(0), V(0), V(0), V(0)};
       int i = 0;
+#pragma unroll 1
       for (; i + 3 < k; i += 4)
 #pragma unroll
         for (int u = 0; u < 4; ++u) t[u] += h[i + u] * qrow(p, sl, qres, i + u, r);
+#pragma unroll 1
       for (; i < k; ++i) t[0] += h[i] * qrow(p, sl, qres, i, r);
       ws[r] += sign * ((t[0] + t[1]) + (t[2] + t[3]));
     }
@@ -613,6 +719,7 @@ __device__ void vel_axpy(const V *qvres, const V *h, int k, V *v, V sign) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (wid < 6) {
     V s = V(0);
+#pragma unroll 1
     for (int i = lane; i < k; i += 32) s += h[i] * qvres[6 * i + wid];
     s = warp_sum(s);
     if (lane == 0) v[wid] += sign * s;
@@ -620,53 +727,70 @@ __device__ void vel_axpy(const V *qvres, const V *h, int k, V *v, V sign) {
   __syncthreads();
 }
 
-// Gram-Schmidt coefficients, spread over the grid: warp w of CTA c sums
-// h_j = sum_c' pd[j * G + c'] + w_vel . Q_j,vel for j = c + P (w + kPW t),
-// into hg[j] (global); lanes l < 6 start from the body term w_vel,l Q_j,vel(l),
-// lanes stride over c', then a fixed shuffle tree.
+// Stage elems values of buf (16-byte aligned) into dst, eight 16-byte loads in
+// flight per thread; no barrier. The buffers are padded to whole vectors.
 template <typename V>
-__device__ void reduce_dots(const PgArgs &p, const V *pd, int k, const V *wv,
-                            const V *qvres, V *hg) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int G = p.g.G;
-  for (int j = p.rank + p.P * wid; j < k; j += p.P * kPW) {
-    V s = lane < 6 ? wv[lane] * qvres[6 * j + lane] : V(0);
-    for (int c = lane; c < G; c += 32) s += __ldcg(pd + (size_t)j * G + c);
-    s = warp_sum(s);
-    if (lane == 0) hg[j] = s;
+__device__ __forceinline__ void stage_wide(const V *buf, int elems, V *dst) {
+  constexpr int W = 16 / (int)sizeof(V);
+  const int n = (elems + W - 1) / W;
+  const int4 *b = reinterpret_cast<const int4 *>(buf);
+  int4 *d = reinterpret_cast<int4 *>(dst);
+#pragma unroll 1
+  for (int q0 = 0; q0 < n; q0 += 8 * kPB) {
+    int4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int q = q0 + u * kPB + (int)threadIdx.x;
+      if (q < n) v[u] = __ldcg(b + q);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int q = q0 + u * kPB + (int)threadIdx.x;
+      if (q < n) d[q] = v[u];
+    }
   }
 }
 
-// The same sums as reduce_dots, h[j] for j < k into shared memory, in every
-// CTA (identical bits: the same order), when the k x G partials fit the
-// staging buffers stg (hb and the partial-sum staging after it): false, with
-// nothing done, otherwise. The partials are staged with eight
-// loads in flight per thread. Ends with a barrier.
-template <typename V>
-__device__ bool local_dots(const PgArgs &p, const V *pd, int k, const V *wv,
-                           const V *qvres, V *h, V *stg) {
-  const int G = p.g.G, tot = k * G;
-  if (tot > kHB * (int)(sizeof(double) / sizeof(V)) + 8 * kMaxPgCtas) return false;
-  for (int q0 = 0; q0 < tot; q0 += 8 * kPB) {
-    V v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int q = q0 + u * kPB + (int)threadIdx.x;
-      v[u] = q < tot ? __ldcg(pd + q) : V(0);
+// The sums of one Gram-Schmidt pass from its partials pd (rows as above), in
+// every CTA (identical bits: the same order): tf[0] = the sum of squares,
+// tf[1..6] = the body sums (SUMS; tf[7] no meaning), h[j], j < k, the dots with the body rows
+// wv. Warp w sums items w + kPW t: lanes l < 6 start a dot from its body term,
+// lanes stride over the CTAs, then a fixed shuffle tree. Partials that don't fit
+// hb (kHB doubles) are summed one dot per warp across the grid, published in hg
+// and read back after a barrier (false: it was abandoned). Ends with a barrier.
+template <bool SUMS, typename V>
+__device__ bool pass_sums(const PgArgs &p, unsigned *epoch, const V *pd, int k, const V *wv,
+                          const V *qvres, V *h, V *tf, double *hb, V *hg) {
+  const int G = p.g.G, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int first = SUMS ? 0 : kSums, all = kSums + k;
+  const bool local = (all - first) * G <= kHB * (int)(sizeof(double) / sizeof(V));
+  V *stg = reinterpret_cast<V *>(hb);
+  const V *pdot = pd + kSums * G;
+  if (!local) {
+#pragma unroll 1
+    for (int j = p.rank + p.P * wid; j < k; j += p.P * kPW) {
+      V s = lane < 6 ? wv[lane] * qvres[6 * j + lane] : V(0);
+#pragma unroll 1
+      for (int c = lane; c < G; c += 32) s += __ldcg(pdot + (size_t)j * G + c);
+      s = warp_sum(s);
+      if (lane == 0) hg[j] = s;
     }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int q = q0 + u * kPB + (int)threadIdx.x;
-      if (q < tot) stg[q] = v[u];
-    }
+    if (!pg_barrier(p, epoch)) return false;
+#pragma unroll 1
+    for (int j = threadIdx.x; j < k; j += kPB) h[j] = __ldcg(hg + j);
   }
+  const int last = local ? all : kSums;
+  const V *rows = SUMS ? pd : pdot;
+  if (last > first) stage_wide(rows, (last - first) * G, stg);
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int j = wid; j < k; j += kPW) {
-    V s = lane < 6 ? wv[lane] * qvres[6 * j + lane] : V(0);
-    for (int c = lane; c < G; c += 32) s += stg[(size_t)j * G + c];
+#pragma unroll 1
+  for (int j = first + wid; j < last; j += kPW) {
+    const V *row = stg + (j - first) * G;
+    V s = j >= kSums && lane < 6 ? wv[lane] * qvres[6 * (j - kSums) + lane] : V(0);
+#pragma unroll 1
+    for (int c = lane; c < G; c += 32) s += row[c];
     s = warp_sum(s);
-    if (lane == 0) h[j] = s;
+    if (lane == 0) (j < kSums ? tf + j : h + (j - kSums))[0] = s;
   }
   __syncthreads();
   return true;
@@ -677,6 +801,7 @@ __device__ bool local_dots(const PgArgs &p, const V *pd, int k, const V *wv,
 // returns |beta_k| / norm_rhs. One thread.
 __device__ double givens_step(int k, double *hcol, double *cs, double *sn, double *beta,
                               double norm_rhs) {
+#pragma unroll 1
   for (int i = 1; i < k; ++i) {
     const double tt = cs[i - 1] * hcol[i - 1] + sn[i - 1] * hcol[i];
     hcol[i] = cs[i - 1] * hcol[i] - sn[i - 1] * hcol[i - 1];
@@ -709,6 +834,7 @@ __device__ void back_substitute(const PgArgs &p, int k, const double *hcol, cons
                                 double *yv, double *hb) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int ld = p.g.max_iter + 1;
+#pragma unroll 1
   for (int i = threadIdx.x; i < k; i += kPB) yv[i] = beta[i];
   int jhi = k - 1;
   while (jhi >= 0) {
@@ -720,7 +846,9 @@ __device__ void back_substitute(const PgArgs &p, int k, const double *hcol, cons
     }
     __syncthreads();
     int off = 0;
+#pragma unroll 1
     for (int j = jhi; j >= jlo; --j) {
+#pragma unroll 1
       for (int i = threadIdx.x; i <= j; i += kPB)
         hb[off + i] = (j == k - 1) ? hcol[i] : ldcg(p.g.H + i + (size_t)j * ld);
       off += j + 1;
@@ -728,9 +856,11 @@ __device__ void back_substitute(const PgArgs &p, int k, const double *hcol, cons
     __syncthreads();
     if (wid == 0) {
       off = 0;
+#pragma unroll 1
       for (int j = jhi; j >= jlo; --j) {
         const double yj = yv[j] / hb[off + j];
         __syncwarp();
+#pragma unroll 1
         for (int i = lane; i < j; i += 32) yv[i] -= hb[off + i] * yj;
         __syncwarp();
         if (lane == 0) yv[j] = yj;
@@ -782,6 +912,8 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
   V *p6 = reinterpret_cast<V *>(p.p6), *ps = reinterpret_cast<V *>(p.ps);
   V *pd1 = reinterpret_cast<V *>(p.pd1), *pd2 = reinterpret_cast<V *>(p.pd2);
 
+  __shared__ float tx[6][kPB];
+  int held = -1;
   const GmresArgs &g = p.g;
   GmresScalars *st = g.st;
   const PSlice sl = pg_slice(p, dsl);
@@ -790,8 +922,11 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
 
   // ---- start: the slice's d_m and the body matrices into shared memory,
   //      warm start into soln, FP32 targets, records, ||rhs|| partials
+#pragma unroll 1
   for (int r = threadIdx.x; r < sl.rows; r += kPB) dsl[r] = V(g.diff[3 * (size_t)sl.m0 + r]);
+#pragma unroll 1
   for (int q = threadIdx.x; q < 72; q += kPB) mats[q] = V(g.mats[q]);
+#pragma unroll 1
   for (int r = threadIdx.x; r < sl.rows; r += kPB) {
     const int t = 3 * sl.m0 + r;
     const double x0 = g.f_blobs[t];
@@ -799,34 +934,37 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
     ws[r] = V(x0);
     zs[r] = V(g.rhs[t]);
   }
+#pragma unroll 1
   for (int m = sl.m0 + threadIdx.x; m < sl.m1; m += kPB)
     for (int k = 0; k < 3; ++k)
       p.x32[3 * (size_t)m + k] = float(g.x_blobs[3 * (size_t)m + k] - g.origin[k]);
   if (sl.body && threadIdx.x < 6) g.soln[vel + threadIdx.x] = g.v_bodies[threadIdx.x];
   __syncthreads();
   if (!p.zero_start) pack_records(p, sl, ws);
-  slice_partials(p, sl, zs, K_RHS, S_RHS);
-  slice_partials(p, sl, ws, K_SOLN, -1);
+  slice_partials(p, sl, zs, p6 + K_RHS * 6 * G, ps + S_RHS * G);
+  slice_partials(p, sl, ws, p6 + K_SOLN * 6 * G, (V *)nullptr);
   if (!pg_barrier(p, &epoch)) return;
 
   // the residual's slots: r0 = rhs with a zero warm start (A 0 = 0: its
   // M_bb, the residual pass and two barriers are skipped)
   const int k_r0 = p.zero_start ? K_RHS : K_R0, s_r0 = p.zero_start ? S_RHS : S_R0;
   if (p.zero_start) {
+#pragma unroll 1
     for (int r = threadIdx.x; r < sl.rows; r += kPB) ws[r] = zs[r];
     __syncthreads();
   } else {
     // ---- M_bb of the warm start
-    mbb_units(p, src);
+    mbb_units(p, src, tx, held);
     if (!pg_barrier(p, &epoch)) return;
 
     // ---- residual r0 = rhs - A soln (slice rows), partials
     if (threadIdx.x < 6) zv[threadIdx.x] = V(g.v_bodies[threadIdx.x]);
     __syncthreads();
     apply_rows(p, sl, zv, ws, hb, acc);  // ws = A soln (blob rows)
+#pragma unroll 1
     for (int r = threadIdx.x; r < sl.rows; r += kPB) ws[r] = zs[r] - ws[r];  // zs = rhs rows
     __syncthreads();
-    slice_partials(p, sl, ws, K_R0, S_R0);
+    slice_partials(p, sl, ws, p6 + K_R0 * 6 * G, ps + S_R0 * G);
     if (!pg_barrier(p, &epoch)) return;
   }
 
@@ -859,6 +997,7 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
     __syncthreads();
     if (flag == 1 || flag == 3) {
       if (flag == 3) {
+#pragma unroll 1
         for (int r = threadIdx.x; r < sl.rows; r += kPB) g.f_blobs[3 * sl.m0 + r] = 0.0;
         if (sl.body && threadIdx.x < 6) g.v_bodies[threadIdx.x] = 0.0;
       }
@@ -876,6 +1015,7 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
     int kslot;
     double inv;
     if (flag == 2) {
+#pragma unroll 1
       for (int r = threadIdx.x; r < sl.rows; r += kPB) {
         ws[r] = zs[r];
         g.soln[3 * sl.m0 + r] = 0.0;
@@ -891,6 +1031,7 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
     }
     const V rinv = V(1.0 / inv);
     __syncthreads();
+#pragma unroll 1
     for (int r = threadIdx.x; r < sl.rows; r += kPB) ws[r] = ws[r] * rinv;
     __syncthreads();
     store_q(p, sl, qres, 0, ws);
@@ -901,7 +1042,7 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
     if (threadIdx.x < 6) qsres[threadIdx.x] = tf[threadIdx.x] * rinv;
     precond(p, sl, ws, qvel, tf, rinv, zs, zv, mats);
     pack_records(p, sl, zs);
-    slice_partials(p, sl, zs, K_Z, -1);
+    slice_partials(p, sl, zs, p6 + K_Z * 6 * G, (V *)nullptr);
   }
   if (!pg_barrier(p, &epoch)) return;
 
@@ -913,11 +1054,12 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
   double qn = 0.0;
   for (;;) {
     PG_STAMP(k, 0);
-    mbb_units(p, src);
+    mbb_units(p, src, tx, held);
     if (p.rank == 0 && k > 1) {
       // Givens rotation (mobility_solver.cpp:2370-2413) of step kk = k - 1
       const int kk = k - 1;
       if (threadIdx.x == 0) {
+#pragma unroll 1
         for (int i = 0; i < kk; ++i) hcol[i] = (double)h1[i] + (double)h2[i];
         hcol[kk] = qn;
         const double rel = givens_step(kk, hcol, cs, sn, beta, norm_rhs);
@@ -933,9 +1075,11 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
       }
       __syncthreads();
       const int ld = g.max_iter + 1;
+#pragma unroll 1
       for (int i = threadIdx.x; i <= kk; i += kPB) g.H[i + (size_t)(kk - 1) * ld] = hcol[i];
       if (tmp8[0] != 0.0) {
         back_substitute(p, kk, hcol, beta, yv, hb);
+#pragma unroll 1
         for (int i = threadIdx.x; i < kk; i += kPB) yg[i] = V(yv[i]);
       }
       if (threadIdx.x == 0) {
@@ -993,62 +1137,54 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
       apply_rows(p, sl, zv, ws, hb, acc);
     }
     if (threadIdx.x < 6) wvel[threadIdx.x] = -tf[threadIdx.x];
+    __syncthreads();
     PG_STAMP(k, 2);
-    slice_dots(p, sl, ws, k, pd1, qres);
+    slice_dots(p, sl, ws, k, pd1 + kSums * G, qres);
     if (!pg_barrier(p, &epoch)) return;
     PG_STAMP(k, 3);
-    // h1 (summed by every CTA while the partials fit the staging buffers,
-    // else spread over the grid and published)
-    V *stg = reinterpret_cast<V *>(hb);
-    if (!local_dots(p, pd1, k, wvel, qvres, h1, stg)) {
-      reduce_dots(p, pd1, k, wvel, qvres, h1g);
-      if (!pg_barrier(p, &epoch)) return;
-      for (int i = threadIdx.x; i < k; i += kPB) h1[i] = __ldcg(h1g + i);
-      __syncthreads();
-    }
+    // h1 (summed by every CTA while the partials fit the staging buffer, else
+    // spread over the grid and published)
+    if (!pass_sums<false>(p, &epoch, pd1, k, wvel, qvres, h1, tf, hb, h1g)) return;
     PG_STAMP(k, 4);
 
     // w' = w - Q h1; CGS pass 2 partial dots, and ||w'||^2 and
     // sum (w' ; d x w') partials
     slice_axpy(p, sl, h1, k, ws, V(-1), qres);
     vel_axpy(qvres, h1, k, wvel, V(-1));
-    slice_dots(p, sl, ws, k, pd2, qres);
-    slice_partials(p, sl, ws, K_W, S_NORM);
+    slice_dots(p, sl, ws, k, pd2 + kSums * G, qres);
+    slice_partials(p, sl, ws, pd2 + G, pd2);
     if (!pg_barrier(p, &epoch)) return;
     PG_STAMP(k, 5);
-    if (!local_dots(p, pd2, k, wvel, qvres, h2, stg)) {
-      reduce_dots(p, pd2, k, wvel, qvres, h2g);
-      if (!pg_barrier(p, &epoch)) return;
-      for (int i = threadIdx.x; i < k; i += kPB) h2[i] = __ldcg(h2g + i);
-      __syncthreads();
-    }
+    if (!pass_sums<true>(p, &epoch, pd2, k, wvel, qvres, h2, tf, hb, h2g)) return;
     PG_STAMP(k, 6);
 
     // w'' = w' - Q h2; with Q orthonormal, ||w''||^2 = ||w'||^2 - ||h2||^2
     // and sum (w'' ; d x w'') = sum (w' ; d x w') - sum_i h2_i S_i, S_i the
     // sums of Q_i (kept in qsres); Q_k = w'' / ||w''||, z_k = P^-1 Q_k.
     // After the first pass h2 is small against w' (the lost orthogonality),
-    // so the difference carries no cancellation.
-    stage(ps + (size_t)S_NORM * G, G, cst);
-    stage(p6 + (size_t)K_W * 6 * G, 6 * G, cst + G);
-    __syncthreads();
-    sum_staged(cst, G, 7, tf);
-    __syncthreads();
+    // so the difference carries no cancellation. Rows on the first warps (four
+    // threads each), the sums and the body rows on the last ones.
     {
-      // warp j < 6: the body sum j of w''; warp 6: ||w''||^2 (lanes over i)
-      const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+      const int lane = threadIdx.x & 31, wid = kPW - 1 - (int)(threadIdx.x >> 5);
       if (wid < 7) {
-        V t = V(0);
+        V t = V(0), q = V(0);
         if (wid < 6) {
-          for (int i = lane; i < k; i += 32) t += h2[i] * qsres[6 * i + wid];
+#pragma unroll 1
+          for (int i = lane; i < k; i += 32) {
+            t += h2[i] * qsres[6 * i + wid];
+            q += h2[i] * qvres[6 * i + wid];
+          }
         } else {
+#pragma unroll 1
           for (int i = lane; i < k; i += 32) t -= h2[i] * h2[i];
           if (lane < 6) t += wvel[lane] * wvel[lane];
         }
         t = warp_sum(t);
+        q = warp_sum(q);
         if (lane == 0) {
           if (wid < 6) {
             wsum6[wid] = tf[1 + wid] - t;
+            qvel[wid] = wvel[wid] - q;
           } else {
             const V w2 = tf[0] + t;
             const V y = vrsqrt(w2);
@@ -1058,23 +1194,32 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
         }
       }
     }
-    __syncthreads();
-    slice_axpy(p, sl, h2, k, ws, V(-1), qres);
-    vel_axpy(qvres, h2, k, wvel, V(-1));
+    slice_axpy(p, sl, h2, k, ws, V(-1), qres);  // ends with a barrier
     qn = qn_s[0];
     const V rqn = qn_s[1];
-    for (int r = threadIdx.x; r < sl.rows; r += kPB) ws[r] = ws[r] * rqn;
-    __syncthreads();
-    store_q(p, sl, qres, k, ws);
-    if (threadIdx.x < 6) {
-      qvel[threadIdx.x] = wvel[threadIdx.x] * rqn;
-      qvres[6 * k + threadIdx.x] = qvel[threadIdx.x];
-      qsres[6 * k + threadIdx.x] = wsum6[threadIdx.x] * rqn;
+    if (threadIdx.x >= kPB - 32) {
+      const int lane = threadIdx.x & 31;
+      if (lane < 6) {
+        qvel[lane] *= rqn;
+        qvres[6 * k + lane] = qvel[lane];
+        qsres[6 * k + lane] = wsum6[lane] * rqn;
+      }
+      __syncwarp();
+      precond_body(qvel, wsum6, rqn, zv, mats);
+    } else {
+#pragma unroll 1
+      for (int r = threadIdx.x; r < sl.rows; r += kPB - 32) {
+        const V q = ws[r] * rqn;
+        ws[r] = q;
+        if (k < p.Kr) qres[(size_t)k * sl.rows + r] = q;
+        else qglobal<V>(p)[(size_t)k * p.g.n + 3 * (size_t)sl.m0 + r] = q;
+      }
     }
     __syncthreads();
-    precond(p, sl, ws, qvel, wsum6, rqn, zs, zv, mats);
+    precond_rows(p, sl, ws, zs, zv);
     pack_records(p, sl, zs);
-    slice_partials(p, sl, zs, K_Z, -1);
+    __syncthreads();
+    slice_partials(p, sl, zs, p6 + K_Z * 6 * G, (V *)nullptr);
     PG_STAMP(k, 7);
     if (!pg_barrier(p, &epoch)) return;
     ++k;
@@ -1082,16 +1227,19 @@ __global__ void __launch_bounds__(kPB, 1) gmres_persistent_kernel(const PgArgs *
 
   // ---- tmp = Q y (slice rows in ws, body rows in qvel), z = P^-1 tmp,
   //      soln += z -> (f_blobs, v_bodies) (:2440-2563)
+#pragma unroll 1
   for (int i = threadIdx.x; i < k; i += kPB) yf[i] = __ldcg(yg + i);
+#pragma unroll 1
   for (int r = threadIdx.x; r < sl.rows; r += kPB) ws[r] = V(0);
   if (threadIdx.x < 6) qvel[threadIdx.x] = V(0);
   __syncthreads();
   slice_axpy(p, sl, yf, k, ws, V(1), qres);
   vel_axpy(qvres, yf, k, qvel, V(1));
-  slice_partials(p, sl, ws, K_T, -1);
+  slice_partials(p, sl, ws, p6 + K_T * 6 * G, (V *)nullptr);
   if (!pg_barrier(p, &epoch)) return;
   cta_sums(p6 + (size_t)K_T * 6 * G, G, 6, tf, cst);
   precond(p, sl, ws, qvel, tf, V(1), zs, zv, mats);
+#pragma unroll 1
   for (int r = threadIdx.x; r < sl.rows; r += kPB) {
     const int t = 3 * sl.m0 + r;
     const double x = g.soln[t] + (double)zs[r];

@@ -112,7 +112,7 @@ __device__ __forceinline__ void flow_pair2(float2 (&v)[3], float2 (&n)[3], float
                                            float2 dz, float2 z2, float2 nz, const float2 (&f)[FD]) {
   const float2 h2 = fma2(dx, dx, mul2(dy, dy));
   const float2 r2 = fma2(dz, dz, h2);
-  const float2 rm1 = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+  const float2 rm1 = make_float2(rsqrt_far(r2.x), rsqrt_far(r2.y));
   const float2 rm3 = mul2(mul2(rm1, rm1), rm1);
   const float2 hF = fma2(dx, f[0], mul2(dy, f[1]));
   const float2 dF = fma2(dz, f[2], hF);
@@ -133,7 +133,7 @@ __device__ __forceinline__ void flow_pair2(float2 (&v)[3], float2 (&n)[3], float
       const float2 sz = mul2(both(-1.f), nz);
       const float2 Rz = add2(z2, sz);
       const float2 R2 = fma2(Rz, Rz, h2);
-      const float2 Rm1 = make_float2(rsqrt_ftz(R2.x), rsqrt_ftz(R2.y));
+      const float2 Rm1 = make_float2(rsqrt_far(R2.x), rsqrt_far(R2.y));
       const float2 Rm2 = mul2(Rm1, Rm1), Rm3 = mul2(Rm1, Rm2);
       const float2 RF = mul2(Rz, f[2]);
       const float2 W = mul2(Rm3, add2(hF, RF));

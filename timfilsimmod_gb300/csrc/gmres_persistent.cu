@@ -436,7 +436,7 @@ __device__ __forceinline__ void mbb_tile(const float (&xt)[2], const float (&yt)
       nf[0] += f0 ? 0u : 1u;
       nf[1] += f1 ? 0u : 1u;
       const float2 rm1 =
-          make_float2(f0 ? rsqrt_ftz(r2.x) : 0.f, f1 ? rsqrt_ftz(r2.y) : 0.f);
+          make_float2(f0 ? rsqrt_far(r2.x) : 0.f, f1 ? rsqrt_far(r2.y) : 0.f);
       // far_pair<float, 3, 3>, operation by operation
       const float2 rm2 = mul2(rm1, rm1), rm3 = mul2(rm1, rm2), rm5 = mul2(rm3, rm2);
       const float2 A = fma2(s, rm3, rm1), B = fma2(s3, rm5, rm3);
@@ -460,7 +460,7 @@ __device__ __forceinline__ void mbb_tile(const float (&xt)[2], const float (&yt)
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
       const bool far = r2 > pc.asum2;
       nf[0] += far ? 0u : 1u;
-      far_pair<float, 3, 3>(v[0], dx, dy, dz, far ? rsqrt_ftz(r2) : 0.f, f, pc);
+      far_pair<float, 3, 3>(v[0], dx, dy, dz, far ? rsqrt_far(r2) : 0.f, f, pc);
     }
   }
   // a target whose only pair inside the contact distance in this tile is

@@ -47,13 +47,6 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
 
-// r^2 of a far pair is a normal number wherever 1/r^3 is finite
-__device__ __forceinline__ float rsqrt_ftz(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <int FD>
 struct Pair2 {
   static constexpr int len = FD == 6 ? 20 : 12;  // floats of two sources
@@ -215,8 +208,8 @@ __device__ __forceinline__ void sum_source_range2(const float (&xt)[TPT], const 
         const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
         rmin[t] = fminf(rmin[t], fminf(r2.x, r2.y));
         float2 rm1;
-        rm1.x = r2.x > pc.asum2 ? rsqrt_ftz(r2.x) : 0.f;
-        rm1.y = r2.y > pc.asum2 ? rsqrt_ftz(r2.y) : 0.f;
+        rm1.x = r2.x > pc.asum2 ? rsqrt_far(r2.x) : 0.f;
+        rm1.y = r2.y > pc.asum2 ? rsqrt_far(r2.y) : 0.f;
         far_pair2<VD, FD>(v[t], dx, dy, dz, rm1, f, s, s3);
       }
     }

@@ -41,7 +41,17 @@ __device__ __forceinline__ double rsqrt_far(double x) {
   return fma(g, p, y0);
 }
 
-__device__ __forceinline__ float rsqrt_far(float x) { return rsqrtf(x); }
+// FP32: the hardware estimate without the range steps of rsqrtf (the same bits
+// for normal x; r^2 of a far pair is a normal number wherever 1/r^3 is finite).
+// Three instructions less of some sixty a 6x6 pair: the plain FP32 products of
+// an implicit step (12 800 segments, 2 562 blobs) 453 -> 414 us. (Two targets in
+// the halves of packed instructions, the same bits again, gain nothing there:
+// 425 us.)
+__device__ __forceinline__ float rsqrt_far(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
 template <typename T>
 __device__ __forceinline__ T sqrt_t(T x);

@@ -69,7 +69,11 @@ cudaError_t launch_queue(int fp32, int variant, int sources, const QueueJob *job
   if (variant < 0 || variant >= nvar) variant = 0;
   if (!fp32) {
     if (ev) cudaEventRecord(ev[0], st);
-    const cudaError_t e = launch_fx(variant, sources, jobs, jobs_host, n_jobs, counters, st);
+    bool taken = false;  // (a pinned variant keeps the tile form)
+    cudaError_t e = cudaSuccess;
+    if (variant == 0) e = launch_plain64(sources, jobs, jobs_host, n_jobs, counters, st, &taken);
+    if (e == cudaSuccess && !taken)
+      e = launch_fx(variant, sources, jobs, jobs_host, n_jobs, counters, st);
     if (ev) cudaEventRecord(ev[1], st);
     return e;
   }

@@ -1,5 +1,5 @@
-// rpy_bb64.cu -- FP64 products of few targets whose sums must keep the bits of
-// the tile form (rpy_chain.cuh): the blob-blob product of the kernel-sequence
+// rpy_bb64.cu -- FP64 products whose sums must keep the bits of the tile form
+// (rpy_chain.cuh): the blob-blob product of the kernel-sequence
 // GMRES and the plain work-queue jobs. A warm-started FP64 GMRES amplifies a
 // difference of 1e-14 in its product up to 1e5 times, so the order of the sums
 // is part of the result.
@@ -11,8 +11,8 @@
 
 namespace tfs {
 
-// rpy_tile_kernel<double, 3, 3, 0, ...> of 128-source tiles. 642 blobs 184 -> 33.6
-// us, 1 289 blobs 177 -> 103 us.
+// rpy_tile_kernel<double, 3, 3, 0, ...> of 128-source tiles. 642 blobs 184 -> 28 us,
+// 1 289 blobs 177 -> 73 us (34 and 103 us without the integer products).
 __global__ void __launch_bounds__(kChainBlock, 2) rpy_bb64_kernel(const TileArgs args, int nt,
                                                                  double a_self) {
   extern __shared__ __align__(16) double bb_smem[];
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kChainBlock, 2) rpy_bb64_kernel(const TileArgs
 }
 
 // Targets per CTA: the fewest FP64 instructions on the busiest SM. A CTA
-// issues, per 128 sources, 20 a target and 4 stages for the pair scalars and
+// issues, per 128 sources, 12 a target and 4 stages for the pair scalars and
 // 256 a chain warp for the sums; its 3 chains a target fill warps of 32 best
 // at 10, 21 or 32 targets, the SMs at a count that divides the targets well.
 static int bb_targets(int n_tgt, int n_src, int chunk, int sms) {
@@ -86,13 +86,12 @@ cudaError_t launch_bb64(const TileArgs &a, int splits, cudaStream_t st) {
 // kPlainTargets targets against one chunk, handed out by a counter; the
 // chunk sums go to the job's partials, and the last unit of 32 targets (the
 // granularity of the job's arrival counters) adds them in chunk order.
+//
+// Every plain FP64 launch takes this form, as it is the faster one at every
+// size: M_ss with M_bs of 640 segments and 642 blobs 629 -> 101 us, M_sb 318 -> 52
+// us, M_bs of 1 289 blobs on 3 587 segments 482 -> 309 us, on 6 000 634 -> 529,
+// of 2 562 on 3 587 799 -> 605.
 // ---------------------------------------------------------------------------
-// The chain form where there are fewer than this many units of 64 targets for
-// two SMs: M_ss with M_bs of 640 segments and 642 blobs (0.4 units an SM) 629 ->
-// 138 us, M_sb 318 -> 56 us, M_bs of 1 289 blobs on 3 587 segments (2.1) 482 ->
-// 426 us, on 6 000 (3.3) 636 -> 728 us: the tile form then fills the SMs, and
-// has no sums to hand over.
-constexpr int kPlainBlocks2 = 5;
 constexpr int kPlainTargets = 16;  // 96 sums of a segment target: three full warps
 
 template <int VD, int FD>
@@ -218,14 +217,13 @@ cudaError_t launch_plain64(int sources, const QueueJob *jobs, const QueueJob *jo
                            unsigned *counters, cudaStream_t st, bool *taken) {
   *taken = false;
   if (sources == Q_SEG_BLOB) return cudaSuccess;
-  long long units = 0, blocks = 0;
+  long long units = 0;
   for (int j = 0; j < n_jobs; ++j) {
     const QueueJob &q = jobs_host[j];
     if (!q.plain) return cudaSuccess;
     units += (long long)((q.n_tgt + kPlainTargets - 1) / kPlainTargets) * q.n_chunks;
-    blocks += (long long)((q.n_tgt + 63) / 64) * q.n_chunks;
   }
-  if (units == 0 || 2 * blocks >= kPlainBlocks2 * (long long)num_sms()) return cudaSuccess;
+  if (units == 0) return cudaSuccess;
   *taken = true;
   const QueueArgs a{jobs, n_jobs, counters};
   return sources == Q_SEG ? plain64_launch<6>(a, units, st) : plain64_launch<3>(a, units, st);

@@ -12,10 +12,13 @@
 // compute those for 32 sources (a lane each) of one target after another into
 // shared memory, and up to three warps, one lane per (target, component), run
 // the ordered sums of the stage before. Their instructions serve 32 sums at
-// once, so the split costs nothing.
+// once, so the split costs nothing. The scalars' plain products run on the
+// integer pipe beside (soft_mul.cuh), which leaves 12 FP64 instructions of 21
+// for the scalars of a 3x3 pair, 14 of 29 of a 6x6 pair.
 #pragma once
 
 #include "rpy_tile.cuh"
+#include "soft_mul.cuh"
 
 namespace tfs {
 
@@ -31,8 +34,9 @@ constexpr int kChainRow = kChainStage + 1;    // doubles; odd, so lanes of diffe
 template <int VD, int FD>
 struct ChainFields {
   static constexpr int n = VD == 6 && FD == 6 ? 10 : VD == 6 || FD == 6 ? 8 : 5;
-  // FP64 instructions of a pair's scalars, and of a sum's step
-  static constexpr int scalars = VD == 6 && FD == 6 ? 28 : VD == 6 || FD == 6 ? 23 : 20;
+  // FP64 instructions of a pair's scalars (beside the integer products), and of a
+  // sum's step
+  static constexpr int scalars = 12 + (VD == 6 && FD == 6 ? 2 : 0);
   static constexpr int steps = VD == 6 && FD == 6 ? 4 : FD == 6 ? 4 : 2;
   static constexpr int forces = VD == 3 && FD == 3 ? 3 : 2 * FD;  // rows: F, T and, negated, again
 };
@@ -49,6 +53,49 @@ struct ChainShared {
   unsigned near[2][kChainMaxTargets][kChainStages];  // by tile parity: sources inside contact
   int next[2];
 };
+
+// far_pair's scalars of target t and this lane's source into o (row doubles
+// from field to field). SOFT: the products on the integer pipe (soft_mul.cuh),
+// which runs beside the FP64 pipe -- 8 of the 20 FP64 instructions of a 3x3
+// pair's scalars and the compare, 15 of 28 of a 6x6 pair's; !ok: one of them is
+// out of its range, and the scalars are to be computed without.
+template <int VD, int FD, bool SOFT>
+__device__ __forceinline__ void pair_scalars(const ChainShared &sh, int t, double sx, double sy,
+                                             double sz, const double (&f)[FD],
+                                             const PairConst<double> &pc, double *o, int row,
+                                             bool &far, bool &ok) {
+  auto mul = [&](double a, double b) { return SOFT ? soft::mul(a, b, &ok) : a * b; };
+  const double dx = sh.xt[0][t] - sx, dy = sh.xt[1][t] - sy, dz = sh.xt[2][t] - sz;
+  const double r2 = fma(dx, dx, fma(dy, dy, mul(dz, dz)));
+  if constexpr (SOFT) {
+    // numbers not below zero compare as their bits do; a NaN is above infinity
+    const long long u = __double_as_longlong(r2);
+    far = u > __double_as_longlong(pc.asum2) && u <= 0x7ff0000000000000ll;
+  } else {
+    far = r2 > pc.asum2;
+  }
+  const double rs = rsqrt_far(r2, mul);
+  const double rm1 = far ? rs : 0.0;
+  const double rm2 = mul(rm1, rm1);
+  const double rm3 = mul(rm1, rm2);
+  const double rm5 = mul(rm3, rm2);
+  const double dF = fma(dx, f[0], fma(dy, f[1], mul(dz, f[2])));
+  o[0] = fma(pc.s, rm3, rm1);
+  o[row] = mul(fma(pc.s3, rm5, rm3), dF);
+  o[2 * row] = dx;
+  o[3 * row] = dy;
+  o[4 * row] = dz;
+  if constexpr (VD == 6 || FD == 6) {
+    o[5 * row] = mul(rm3, dx);
+    o[6 * row] = mul(rm3, dy);
+    o[7 * row] = mul(rm3, dz);
+  }
+  if constexpr (VD == 6 && FD == 6) {
+    const double dT = fma(dx, f[3], fma(dy, f[4], mul(dz, f[5])));
+    o[8 * row] = mul(-0.5, rm3);
+    o[9 * row] = mul(mul(1.5, rm5), dT);
+  }
+}
 
 // The sum of the lane's (target, component) -- target threadIdx.x / VD, component
 // threadIdx.x % VD, for threadIdx.x < VD cnt -- over the sources [s0, s1) of rec.
@@ -154,32 +201,12 @@ __device__ __forceinline__ double chain_sums(ChainShared &sh, const double *__re
       int t = lane == 0 ? atomicAdd(&sh.next[s & 1], 1) : 0;
       t = __shfl_sync(0xffffffffu, t, 0);
       if (t >= cnt) break;
-      // far_pair, its scalars
-      const double dx = sh.xt[0][t] - sx, dy = sh.xt[1][t] - sy, dz = sh.xt[2][t] - sz;
-      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-      const bool far = r2 > pc.asum2;
-      const double rs = rsqrt_far(r2);
-      const double rm1 = far ? rs : 0.0;
-      const double rm2 = rm1 * rm1;
-      const double rm3 = rm1 * rm2;
-      const double rm5 = rm3 * rm2;
-      const double dF = fma(dx, f[0], fma(dy, f[1], dz * f[2]));
       double *o = buf + t * kChainRow + lane;
-      o[0] = fma(pc.s, rm3, rm1);
-      o[row] = fma(pc.s3, rm5, rm3) * dF;
-      o[2 * row] = dx;
-      o[3 * row] = dy;
-      o[4 * row] = dz;
-      if constexpr (VD == 6 || FD == 6) {
-        o[5 * row] = rm3 * dx;
-        o[6 * row] = rm3 * dy;
-        o[7 * row] = rm3 * dz;
-      }
-      if constexpr (VD == 6 && FD == 6) {
-        const double dT = fma(dx, f[3], fma(dy, f[4], dz * f[5]));
-        o[8 * row] = -0.5 * rm3;
-        o[9 * row] = (1.5 * rm5) * dT;
-      }
+      bool far, ok = true;
+      pair_scalars<VD, FD, true>(sh, t, sx, sy, sz, f, pc, o, row, far, ok);
+      // (a near pair has zero scalars, which the integer products take too)
+      if (__any_sync(0xffffffffu, !ok && j < s1))
+        pair_scalars<VD, FD, false>(sh, t, sx, sy, sz, f, pc, o, row, far, ok);
       const unsigned m = __ballot_sync(0xffffffffu, !far && j < s1);
       if (lane == 0) sh.near[(s / kChainStages) & 1][t][s % kChainStages] = m;
     }

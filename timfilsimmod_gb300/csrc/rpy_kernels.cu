@@ -515,7 +515,7 @@ cudaError_t launch_tile(const TileArgs &a_in, int vd, int fda, int fdb, TileTuni
   if (partials) *partials = splits;
   a.chunk = chunk;
   const dim3 grid(ctas, splits);
-  // the same sums, split further and faster at every size (rpy_bb64.cu: 184 -> 34 us
+  // the same sums, split further and faster at every size (rpy_bb64.cu: 184 -> 28 us
   // at 642 blobs); the other variants stay for the autotuner
   const bool bb64 = !a.fp32 && combo == C_BB && tune.variant == 0;
   cudaError_t e;

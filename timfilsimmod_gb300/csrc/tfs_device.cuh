@@ -28,17 +28,22 @@ constexpr double kPi = 3.14159265358979323846264338327950288;
 // Valid for x in the FP32 normal range [1.2e-38, 1.7e38] (far-field r^2 of
 // any physical configuration); the kernels never call it for r^2 = 0.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double rsqrt_far(double x) {
+// mul: how its two plain products are formed.
+template <typename Mul>
+__device__ __forceinline__ double rsqrt_far(double x, Mul mul) {
   const int hi = __double2hiint(x);
   const float xf = __int_as_float((hi - (896 << 20)) << 3);
   const float yf = rsqrtf(xf);
   const int fb = __float_as_int(yf);
   const double y0 = __hiloint2double((fb >> 3) + (896 << 20), fb << 29);
-  const double t = x * y0;
+  const double t = mul(x, y0);
   const double e = fma(-t, y0, 1.0);
   const double p = fma(e, 0.375, 0.5);
-  const double g = y0 * e;
+  const double g = mul(y0, e);
   return fma(g, p, y0);
+}
+__device__ __forceinline__ double rsqrt_far(double x) {
+  return rsqrt_far(x, [](double a, double b) { return a * b; });
 }
 
 // FP32: the hardware estimate without the range steps of rsqrtf (the same bits

@@ -249,8 +249,8 @@ cudaError_t launch_tile(const TileArgs &a, int vd, int fda, int fdb, TileTuning 
 // rpy_bb64.cu: rpy_tile_kernel<double, 3, 3, 0, ...> of 128-source tiles, bit
 // for bit, for the chunk size, splits, mode and output given.
 cudaError_t launch_bb64(const TileArgs &a, int splits, cudaStream_t st);
-// Plain FP64 work-queue jobs of few targets (*taken: the launch is theirs), the
-// sums of queue_unit<double, ...> bit for bit.
+// Plain FP64 work-queue jobs (*taken: they are, and launched), the sums of
+// queue_unit<double, ...> bit for bit.
 cudaError_t launch_plain64(int sources, const QueueJob *jobs, const QueueJob *jobs_host, int n_jobs,
                            unsigned *counters, cudaStream_t st, bool *taken);
 cudaError_t launch_barrier(const BarrierArgs &a, cudaStream_t st);

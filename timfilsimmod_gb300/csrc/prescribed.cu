@@ -55,6 +55,7 @@ constexpr int kPW = kPT / 32;    // warps per CTA
 constexpr int kGT = 256;
 constexpr int kGW = kGT / 32;
 constexpr int kFilC = 16;        // per-filament constants (below)
+constexpr int kPresMinRows = 128;  // rows of a CTA of the GMRES vector kernels
 constexpr int kPresMaxIter = 350;  // MAX_LINEAR_SYSTEM_ITER (config.hpp:312)
 constexpr int kPresChunk = 4;      // Arnoldi steps launched between polls of the done flag
 // FP32C: the deepest relative reduction an inner solve is asked for. Its
@@ -688,9 +689,9 @@ __global__ void __launch_bounds__(kPT) pres_combine_kernel(PA a, const double *z
   }
   if (!a.free_body) return;
   const int W = a.fil_warps + a.blob_warps;
-  for (int k = 0; k < 6; ++k) p6[k] = pw_sum(p6[k]);
-  if (lane == 0 && w < W)
-    for (int k = 0; k < 6; ++k) a.part6[6 * (size_t)w + k] = p6[k];
+  const double p8[8] = {p6[0], p6[1], p6[2], p6[3], p6[4], p6[5], 0.0, 0.0};
+  const double ps = pw_sum8(p8);
+  if ((lane & 3) == 0 && lane < 24 && w < W) a.part6[6 * (size_t)w + (lane >> 2)] = ps;
   if (!pres_last_cta(a.cnt)) return;
   sum_part6_warps(a, sh);
   if (threadIdx.x < 6) {
@@ -805,22 +806,18 @@ __global__ void __launch_bounds__(kPT) pres_precond_a_kernel(PA a, const double 
   }
   if (!a.free_body) return;
   const int W = a.fil_warps + a.blob_warps;
-  for (int k = 0; k < 6; ++k) p6[k] = pw_sum(p6[k]);
-  if (lane == 0 && w < W)
-    for (int k = 0; k < 6; ++k) a.part6[6 * (size_t)w + k] = p6[k];
+  const double p8[8] = {p6[0], p6[1], p6[2], p6[3], p6[4], p6[5], 0.0, 0.0};
+  const double ps = pw_sum8(p8);
+  if ((lane & 3) == 0 && lane < 24 && w < W) a.part6[6 * (size_t)w + (lane >> 2)] = ps;
   if (!pres_last_cta(a.cnt)) return;
   sum_part6_warps(a, sh);
-  if (threadIdx.x == 0) {
-    double t[6], B[6];
-    for (int k = 0; k < 6; ++k) t[k] = -in[a.o_body + k] - sh[k];
-    for (int r = 0; r < 6; ++r) {
-      double v = 0.0;
-      for (int k = 0; k < 6; ++k) v += a.m6inv[r + 6 * k] * t[k];
-      B[r] = v;
-    }
-    for (int k = 0; k < 6; ++k) out[a.o_body + k] = B[k];
-    *a.cnt = 0u;
+  if (threadIdx.x < 6) {
+    double v = 0.0;
+    for (int k = 0; k < 6; ++k)
+      v += a.m6inv[threadIdx.x + 6 * k] * (-in[a.o_body + k] - sh[k]);
+    out[a.o_body + threadIdx.x] = v;
   }
+  if (threadIdx.x == 0) *a.cnt = 0u;
 }
 
 // Pass B (free body): the phase/angle rows' correction by the body block B
@@ -989,46 +986,56 @@ __global__ void pres_q0_kernel(GA g, const double *rhs, double *x) {
   }
 }
 
-// Dots <w, Q_i>, i < k, over this CTA's rows into part[cta][i]: columns in
-// blocks of 8, every thread accumulating its rows' products for the 8 at once
-// (coalesced row loads; two rows a thread at a time, sixteen loads in
-// flight, each row's products added in row order), block sums per column;
-// the last CTA sums the partials in a fixed order into h, four columns a warp
-// at a time.
+// Dots <w, Q_i>, i < k, over this CTA's rows into part[cta][i]: kDotRows threads
+// over the rows in each of kDotGroups groups, which take the columns in turn,
+// eight at a time (coalesced row loads; two rows a thread at a time, sixteen
+// loads in flight, each row's products added in row order), block sums per
+// column; the last CTA sums the partials in a fixed order into h, four columns
+// a warp at a time.
+//
+// Each SM's FP64 pipe bounds this: few row threads of many rows each spend
+// least on the warp sums (nine adds a warp for eight columns). 64 threads of
+// five rows and four column groups, against 256 threads of one or two rows and
+// the columns in sequence: 4 600 unknowns (52 steps) 29.2 -> 17.7 us for both
+// passes.
+constexpr int kDotRows = 64, kDotGroups = kGT / kDotRows;
 __device__ void pres_dots(const GA &g, const double *w, int k, double *h) {
-  __shared__ double red[kGW][8];
+  __shared__ double red[kDotGroups][kDotRows / 32][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int x = threadIdx.x % kDotRows, group = threadIdx.x / kDotRows;
   const int r0 = blockIdx.x * g.rows, r1 = min(g.n, r0 + g.rows);
-  const int bd = blockDim.x;
-  for (int i0 = 0; i0 < k; i0 += 8) {
-    const int nc = min(8, k - i0);
-    double acc[8];
+  for (int base = 0; base < k; base += 8 * kDotGroups) {
+    const int i0 = base + 8 * group, nc = min(8, k - i0);
+    if (nc > 0) {
+      double acc[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.0;
-    for (int r = r0 + threadIdx.x; r < r1; r += 2 * bd) {
-      const bool two = r + bd < r1;
-      const double wr = w[r], wr2 = two ? w[r + bd] : 0.0;
-      const double *q = g.Q + (size_t)i0 * g.n + r;
-      double a[8], b[8];
+      for (int j = 0; j < 8; ++j) acc[j] = 0.0;
+      for (int r = r0 + x; r < r1; r += 2 * kDotRows) {
+        const bool two = r + kDotRows < r1;
+        const double wr = w[r], wr2 = two ? w[r + kDotRows] : 0.0;
+        const double *q = g.Q + (size_t)i0 * g.n + r;
+        double a[8], b[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        a[j] = j < nc ? q[(size_t)j * g.n] : 0.0;
-        b[j] = (j < nc && two) ? q[(size_t)j * g.n + bd] : 0.0;
+        for (int j = 0; j < 8; ++j) {
+          a[j] = j < nc ? q[(size_t)j * g.n] : 0.0;
+          b[j] = (j < nc && two) ? q[(size_t)j * g.n + kDotRows] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j < nc) acc[j] += a[j] * wr;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j < nc && two) acc[j] += b[j] * wr2;
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (j < nc) acc[j] += a[j] * wr;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (j < nc && two) acc[j] += b[j] * wr2;
+      const double sc = pw_sum8(acc);
+      if ((lane & 3) == 0) red[group][x >> 5][lane >> 2] = sc;
     }
-    const double sc = pw_sum8(acc);
-    if ((lane & 3) == 0) red[wid][lane >> 2] = sc;
     __syncthreads();
-    if ((int)threadIdx.x < nc) {
+    if ((int)threadIdx.x < min(8 * kDotGroups, k - base)) {
       double t = 0.0;
-      for (int q = 0; q < kGW; ++q) t += red[q][threadIdx.x];
-      g.part[(size_t)blockIdx.x * g.pstride + i0 + threadIdx.x] = t;
+#pragma unroll
+      for (int q = 0; q < kDotRows / 32; ++q) t += red[threadIdx.x >> 3][q][threadIdx.x & 7];
+      g.part[(size_t)blockIdx.x * g.pstride + base + threadIdx.x] = t;
     }
     __syncthreads();
   }
@@ -1042,19 +1049,15 @@ __device__ void pres_dots(const GA &g, const double *w, int k, double *h) {
   if (threadIdx.x == 0) *g.cnt = 0u;
 }
 
-// w -= sum_i h_i Q_i over this CTA's rows (h staged in shared memory; the
-// columns of a row subtracted in order; two rows a thread at a time, sixteen
-// loads in flight).
-__device__ void pres_orth(const GA &g, double *w, int k, const double *h) {
-  __shared__ double hs[kPresMaxIter];
-  for (int i = threadIdx.x; i < k; i += blockDim.x) hs[i] = h[i];
-  __syncthreads();
+// w -= sum_i h_i Q_i over this CTA's rows, by kGT threads (h in shared memory;
+// the columns of a row subtracted in order; two rows a thread at a time,
+// sixteen loads in flight). No barrier.
+__device__ void pres_orth(const GA &g, double *w, int k, const double *hs) {
   const int r0 = blockIdx.x * g.rows, r1 = min(g.n, r0 + g.rows);
-  const int bd = blockDim.x;
   const size_t n = g.n;
-  for (int r = r0 + threadIdx.x; r < r1; r += 2 * bd) {
-    const bool two = r + bd < r1;
-    double t = w[r], u = two ? w[r + bd] : 0.0;
+  for (int r = r0 + threadIdx.x; r < r1; r += 2 * kGT) {
+    const bool two = r + kGT < r1;
+    double t = w[r], u = two ? w[r + kGT] : 0.0;
     const double *q = g.Q + r;
     int i = 0;
     for (; i + 8 <= k; i += 8) {
@@ -1062,21 +1065,22 @@ __device__ void pres_orth(const GA &g, double *w, int k, const double *h) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         a[j] = q[(size_t)(i + j) * n];
-        b[j] = two ? q[(size_t)(i + j) * n + bd] : 0.0;
+        b[j] = two ? q[(size_t)(i + j) * n + kGT] : 0.0;
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) t -= hs[i + j] * a[j];
+      if (two) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) u -= hs[i + j] * b[j];
+        for (int j = 0; j < 8; ++j) u -= hs[i + j] * b[j];
+      }
     }
     for (; i < k; ++i) {
       t -= hs[i] * q[(size_t)i * n];
-      if (two) u -= hs[i] * q[(size_t)i * n + bd];
+      if (two) u -= hs[i] * q[(size_t)i * n + kGT];
     }
     w[r] = t;
-    if (two) w[r + bd] = u;
+    if (two) w[r + kGT] = u;
   }
-  __syncthreads();
 }
 
 // Step k = st->iter, pass 1: h1 = Q^T w. (The step kernels read k from the
@@ -1093,29 +1097,60 @@ __global__ void __launch_bounds__(kGT) pres_dots2_kernel(GA g) {
   if (g.st->done) return;
   const int k = g.st->iter;
   double *w = g.Q + (size_t)k * g.n;
-  pres_orth(g, w, k, g.h1);
+  __shared__ double hs[kPresMaxIter];
+  for (int i = threadIdx.x; i < k; i += kGT) hs[i] = g.h1[i];
+  __syncthreads();
+  pres_orth(g, w, k, hs);
+  __syncthreads();
   pres_dots(g, w, k, g.h2);
 }
 
 // Step k: w -= Q h2, ||w||; the last CTA writes H(:, k-1), applies the
 // earlier Givens rotations and the new one (mobility_solver.cpp:2370-2404),
 // tests convergence (:2409-2413) and, when finishing, back-solves y (:2419-
-// 2438) with warp-parallel inner sums. The column and the rotations are
-// staged in shared memory for the serial rotation chain.
-__global__ void __launch_bounds__(kGT) pres_norm_givens_kernel(GA g) {
+// 2438) with warp-parallel inner sums. A ninth warp turns the column by the
+// earlier rotations meanwhile (in shared memory): that needs no norm, and its
+// chain is as long as the projection of the rows.
+__global__ void __launch_bounds__(kGT + 32) pres_norm_givens_kernel(GA g) {
   __shared__ double red[kGW];
-  __shared__ double hc[kPresMaxIter + 1], css[kPresMaxIter], sns[kPresMaxIter];
+  __shared__ double hs[kPresMaxIter];
+  __shared__ double hc[kPresMaxIter + 1], css[kPresMaxIter], sns[kPresMaxIter], tr[kPresMaxIter];
   __shared__ int fin;
   if (g.st->done) return;
-  const int k = g.st->iter;
-  double *w = g.Q + (size_t)k * g.n;
-  pres_orth(g, w, k, g.h2);
+  const int k = g.st->iter, ld = g.ld, c = k - 1;
+  double *w = g.Q + (size_t)k * g.n, *H = g.H;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int r0 = blockIdx.x * g.rows, r1 = min(g.n, r0 + g.rows);
-  double t = 0.0;
-  for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) t += w[r] * w[r];
-  t = pw_sum(t);
-  if (lane == 0) red[wid] = t;
+  for (int i = threadIdx.x; i < k; i += kGT + 32) hs[i] = g.h2[i];
+  __syncthreads();
+  if (wid == kGW) {
+    for (int i = lane; i < k; i += 32) {
+      hc[i] = g.h1[i] + hs[i];
+      if (i < c) {
+        css[i] = g.cs[i];
+        sns[i] = g.sn[i];
+      }
+    }
+    __syncwarp();
+    // tr[i]: entry i turned by rotation i - 1, before rotation i
+    double v = hc[0];
+    for (int i = 1; i < k; ++i) {
+      const double u = css[i - 1] * hc[i] - sns[i - 1] * v;
+      if (lane == 0) tr[i - 1] = v;
+      v = u;
+    }
+    __syncwarp();
+    for (int i = lane; i < c; i += 32) css[i] = css[i] * tr[i] + sns[i] * hc[i + 1];
+    __syncwarp();
+    for (int i = lane; i < c; i += 32) hc[i] = css[i];
+    if (lane == 0) hc[c] = v;
+  } else {
+    pres_orth(g, w, k, hs);
+    const int r0 = blockIdx.x * g.rows, r1 = min(g.n, r0 + g.rows);
+    double t = 0.0;  // (the rows this thread has just written)
+    for (int r = r0 + threadIdx.x; r < r1; r += kGT) t += w[r] * w[r];
+    t = pw_sum(t);
+    if (lane == 0) red[wid] = t;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     double u = 0.0;
@@ -1123,29 +1158,13 @@ __global__ void __launch_bounds__(kGT) pres_norm_givens_kernel(GA g) {
     g.part[(size_t)blockIdx.x * g.pstride] = u;
   }
   if (!pres_last_cta(g.cnt)) return;
-  const int ld = g.ld, c = k - 1;
-  double *H = g.H;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) {
-    hc[i] = g.h1[i] + g.h2[i];
-    if (i < c) {
-      css[i] = g.cs[i];
-      sns[i] = g.sn[i];
-    }
-  }
   double ss = 0.0;
   if (wid == 0) ss = pw_sum_strided(g.part, g.G, g.pstride);
-  __syncthreads();
   PresScalars *st = g.st;
   if (threadIdx.x == 0) {
     const double qn = sqrt(ss);
     st->qnorm = qn;
     hc[k] = qn;
-    for (int i = 1; i < k; ++i) {
-      const double a0 = hc[i - 1], a1 = hc[i];
-      const double tt = css[i - 1] * a0 + sns[i - 1] * a1;
-      hc[i] = css[i - 1] * a1 - sns[i - 1] * a0;
-      hc[i - 1] = tt;
-    }
     const double hk = hc[k], hd = hc[c];
     double cs, sn;
     if (hk == 0.0) {
@@ -1177,7 +1196,7 @@ __global__ void __launch_bounds__(kGT) pres_norm_givens_kernel(GA g) {
     *g.cnt = 0u;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i <= k; i += blockDim.x) H[i + (size_t)c * ld] = hc[i];
+  for (int i = threadIdx.x; i <= k; i += kGT + 32) H[i + (size_t)c * ld] = hc[i];
   __syncthreads();
   if (!fin || wid != 0) return;
   // y(k-1) = beta / H, then upward: y(i) = (beta(i) - sum_{j>i} H(i,j) y(j)) / H(i,i)
@@ -1349,12 +1368,15 @@ int pres_alloc(tfs_solver *s) {
   PresState *p = s->pres;
   const size_t n = p->n, ns = p->ns, nb = p->nb, nf = p->nfil;
   const int ld = kPresMaxIter + 1;
-  // GMRES vector kernels: CTAs of at least 256 consecutive rows; up to one
-  // per SM as the rows allow, beyond that a multiple of the SM count (at most
-  // eight per SM). Each SM's FP64 pipe bounds these kernels on this part, so
-  // every SM gets the same share of the rows.
+  // GMRES vector kernels: CTAs of at least kPresMinRows consecutive rows; up to
+  // one per SM as the rows allow, beyond that a multiple of the SM count (at
+  // most eight per SM), of at least 256 rows (4 600 unknowns, a step's three
+  // kernels with 256, 128 and 64: 34.6, 29.7 and 30.3 us). Each SM's FP64 pipe bounds these
+  // kernels on this part, so every SM gets the same share of the rows.
   const size_t sms = (size_t)num_sms(), g0 = (n + 255) / 256;
-  p->G = (int)std::max<size_t>(1, g0 <= sms ? g0 : std::min<size_t>(8 * sms, g0 / sms * sms));
+  p->G = (int)std::max<size_t>(
+      1, g0 <= sms ? std::min<size_t>(sms, (n + kPresMinRows - 1) / kPresMinRows)
+                   : std::min<size_t>(8 * sms, g0 / sms * sms));
   p->rows = (int)((n + p->G - 1) / p->G);
   p->pstride = kPresMaxIter + 2;
   const size_t warps = nf + (nb + 31) / 32;
@@ -1610,7 +1632,7 @@ int pres_chunk(tfs_solver *s, int fp32) {
     if ((rc = pres_operator(s, fp32, p->z, nullptr, p->Q, p->st)) != TFS_OK) return rc;
     pres_dots1_kernel<<<g.G, kGT, 0, s->stream>>>(g);
     pres_dots2_kernel<<<g.G, kGT, 0, s->stream>>>(g);
-    pres_norm_givens_kernel<<<g.G, kGT, 0, s->stream>>>(g);
+    pres_norm_givens_kernel<<<g.G, kGT + 32, 0, s->stream>>>(g);
     pres_scale_kernel<<<g.G, kGT, 0, s->stream>>>(g);
     count_launch_n(4);
     TFS_CUDA(cudaGetLastError(), "prescribed Arnoldi step");

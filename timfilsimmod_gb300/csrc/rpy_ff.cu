@@ -35,6 +35,7 @@
 #include <cmath>
 
 #include "ff_arith.cuh"
+#include "tfs_device.cuh"
 #include "tfs_kernels.h"
 
 namespace tfs {
@@ -79,10 +80,19 @@ struct FFArgs {
   double *out;           // [gridDim.y][n][3]
 };
 
-// One pair into v (units of 1/(8 pi mu)).
-__device__ __forceinline__ void ff_pair(FF (&v)[3], const FF (&xt)[3], const FF (&xs)[3],
-                                        const FF (&f)[3], const FFConst &k) {
-  const FF dx = ff_sub(xt[0], xs[0]), dy = ff_sub(xt[1], xs[1]), dz = ff_sub(xt[2], xs[2]);
+// The scalars of one pair, far form: d, r^2, 1/r and the coefficients A and B.
+// No branch: a pair at or inside contact is put right by ff_near.
+struct FFPair {
+  FF dx, dy, dz, r2, rm1, A, B;
+  bool far;
+};
+__device__ __forceinline__ FFPair ff_scalars(const FF (&xt)[3], const FF (&xs)[3],
+                                             const FFConst &k) {
+  FFPair p;
+  p.dx = ff_sub(xt[0], xs[0]);
+  p.dy = ff_sub(xt[1], xs[1]);
+  p.dz = ff_sub(xt[2], xs[2]);
+  const FF dx = p.dx, dy = p.dy, dz = p.dz;
   // r^2 (all terms positive)
   const float px = __fmul_rn(dx.h, dx.h), py = __fmul_rn(dy.h, dy.h), pz = __fmul_rn(dz.h, dz.h);
   const float ex = fmaf(__fadd_rn(dx.h, dx.h), dx.l, fmaf(dx.h, dx.h, -px));
@@ -91,42 +101,57 @@ __device__ __forceinline__ void ff_pair(FF (&v)[3], const FF (&xt)[3], const FF 
   FF r2 = ff_two_sum(px, py);
   const float t = __fadd_rn(r2.l, __fadd_rn(ex, ey));
   r2 = ff_two_sum(r2.h, pz);
-  r2 = ff_fast_two_sum(r2.h, __fadd_rn(r2.l, __fadd_rn(t, ez)));
-  FF A, B;
-  const bool far = r2.h > k.asum2.h || (r2.h == k.asum2.h && r2.l > k.asum2.l);
-  if (r2.h == 0.f) {  // self
-    A = k.self;
-    B = {0.f, 0.f};
-  } else {
-    // 1/r
-    const float y0 = rsqrtf(r2.h);
-    const float qh = __fmul_rn(y0, y0);
-    const float ql = fmaf(y0, y0, -qh);
-    const float uh = __fmul_rn(r2.h, qh);
-    const float ul = fmaf(r2.h, ql, fmaf(r2.l, qh, fmaf(r2.h, qh, -uh)));
-    const float e = __fsub_rn(__fsub_rn(1.0f, uh), ul);
-    const float c = __fmul_rn(__fmul_rn(y0, e), fmaf(e, 0.375f, 0.5f));
-    const FF rm1 = ff_fast_two_sum(y0, c);
-    if (far) {
-      const FF rm2 = ff_mul(rm1, rm1);
-      const FF rm3 = ff_mul(rm1, rm2);
-      const FF rm5 = ff_mul(rm3, rm2);
-      A = ff_add(rm1, ff_mul(k.s, rm3));
-      B = ff_add(rm3, ff_mul(k.s3, rm5));
-    } else {
-      const FF r = ff_mul(r2, rm1);
-      A = ff_add(k.self, ff_mul(k.near_r, r));
-      B = ff_mul(k.near_d, rm1);
-    }
+  p.r2 = r2 = ff_fast_two_sum(r2.h, __fadd_rn(r2.l, __fadd_rn(t, ez)));
+  p.far = r2.h > k.asum2.h || (r2.h == k.asum2.h && r2.l > k.asum2.l);
+  // 1/r
+  const float y0 = rsqrt_far(r2.h);
+  const float qh = __fmul_rn(y0, y0);
+  const float ql = fmaf(y0, y0, -qh);
+  const float uh = __fmul_rn(r2.h, qh);
+  const float ul = fmaf(r2.h, ql, fmaf(r2.l, qh, fmaf(r2.h, qh, -uh)));
+  const float e = __fsub_rn(__fsub_rn(1.0f, uh), ul);
+  const float c = __fmul_rn(__fmul_rn(y0, e), fmaf(e, 0.375f, 0.5f));
+  p.rm1 = ff_fast_two_sum(y0, c);
+  const FF rm2 = ff_mul(p.rm1, p.rm1);
+  const FF rm3 = ff_mul(p.rm1, rm2);
+  const FF rm5 = ff_mul(rm3, rm2);
+  p.A = ff_add(p.rm1, ff_mul(k.s, rm3));
+  p.B = ff_add(rm3, ff_mul(k.s3, rm5));
+  return p;
+}
+
+// The coefficients of a pair at or inside contact.
+__device__ __forceinline__ void ff_near(FFPair &p, const FFConst &k) {
+  if (p.r2.h == 0.f) {  // self
+    p.A = k.self;
+    p.B = {0.f, 0.f};
+    return;
   }
-  const FF dF = ff_add(ff_add(ff_mul(dx, f[0]), ff_mul(dy, f[1])), ff_mul(dz, f[2]));
-  const FF Bd = ff_mul(B, dF);
-  ff_acc(v[0], ff_mul(A, f[0]));
-  ff_acc(v[0], ff_mul(Bd, dx));
-  ff_acc(v[1], ff_mul(A, f[1]));
-  ff_acc(v[1], ff_mul(Bd, dy));
-  ff_acc(v[2], ff_mul(A, f[2]));
-  ff_acc(v[2], ff_mul(Bd, dz));
+  // (1/r by rsqrtf: r^2 may be subnormal here)
+  const FF r2 = p.r2;
+  const float y0 = rsqrtf(r2.h);
+  const float qh = __fmul_rn(y0, y0);
+  const float ql = fmaf(y0, y0, -qh);
+  const float uh = __fmul_rn(r2.h, qh);
+  const float ul = fmaf(r2.h, ql, fmaf(r2.l, qh, fmaf(r2.h, qh, -uh)));
+  const float e = __fsub_rn(__fsub_rn(1.0f, uh), ul);
+  const float c = __fmul_rn(__fmul_rn(y0, e), fmaf(e, 0.375f, 0.5f));
+  const FF rm1 = ff_fast_two_sum(y0, c);
+  const FF r = ff_mul(r2, rm1);
+  p.A = ff_add(k.self, ff_mul(k.near_r, r));
+  p.B = ff_mul(k.near_d, rm1);
+}
+
+// The pair into v (units of 1/(8 pi mu)).
+__device__ __forceinline__ void ff_add_pair(FF (&v)[3], const FFPair &p, const FF (&f)[3]) {
+  const FF dF = ff_add(ff_add(ff_mul(p.dx, f[0]), ff_mul(p.dy, f[1])), ff_mul(p.dz, f[2]));
+  const FF Bd = ff_mul(p.B, dF);
+  ff_acc(v[0], ff_mul(p.A, f[0]));
+  ff_acc(v[0], ff_mul(Bd, p.dx));
+  ff_acc(v[1], ff_mul(p.A, f[1]));
+  ff_acc(v[1], ff_mul(Bd, p.dy));
+  ff_acc(v[2], ff_mul(p.A, f[2]));
+  ff_acc(v[2], ff_mul(Bd, p.dz));
 }
 
 // grid = (target CTAs, source splits); BLOCK threads, TPT targets each;
@@ -158,8 +183,20 @@ __global__ void __launch_bounds__(BLOCK) bb_ff_kernel(const FFArgs a) {
       const float4 r0 = src[3 * j], r1 = src[3 * j + 1], r2 = src[3 * j + 2];
       const FF xs[3] = {{r0.x, r1.z}, {r0.y, r1.w}, {r0.z, r2.x}};
       const FF f[3] = {{r0.w, r2.y}, {r1.x, r2.z}, {r1.y, r2.w}};
+      FFPair p[TPT];
+      bool near = false;
 #pragma unroll
-      for (int t = 0; t < TPT; ++t) ff_pair(v[t], xt[t], xs, f, a.k);
+      for (int t = 0; t < TPT; ++t) {
+        p[t] = ff_scalars(xt[t], xs, a.k);
+        near = near || !p[t].far;
+      }
+      if (__any_sync(0xffffffffu, near)) {
+#pragma unroll
+        for (int t = 0; t < TPT; ++t)
+          if (!p[t].far) ff_near(p[t], a.k);
+      }
+#pragma unroll
+      for (int t = 0; t < TPT; ++t) ff_add_pair(v[t], p[t], f);
     }
   }
 #pragma unroll
@@ -172,7 +209,11 @@ __global__ void __launch_bounds__(BLOCK) bb_ff_kernel(const FFArgs a) {
   }
 }
 
-constexpr int kFFBlock = 128, kFFTpt = 2, kFFTs = 128;
+// One target a thread and no branch in a pair (but for contact, once a warp):
+// 2 562 blobs 67-81 -> 63 us, 15 362 2 234 -> 1 770 us. Two targets a thread:
+// 70-81 and 1 738-2 141 us.
+constexpr int kFFBlock = 128, kFFTpt = 1, kFFTs = 128;
+constexpr int kFFSplitTargets = 256;  // targets a CTA that the splits count with
 
 FF host_split(double x) {
   const float h = (float)x;
@@ -207,8 +248,9 @@ cudaError_t launch_bb_ff(const double *x_blobs, const double *f_blobs, int nb,
   a.k.near_d = host_split(1.0 / (8.0 * a2));
   // source splits: about four CTAs per SM in all, sources per split a
   // multiple of the tile, partial sums within the scratch
+  const int split_ctas = (nb + kFFSplitTargets - 1) / kFFSplitTargets;
   const int ctas = (nb + kFFBlock * kFFTpt - 1) / (kFFBlock * kFFTpt);
-  int splits = std::max(1, (4 * num_sms() + ctas - 1) / ctas);
+  int splits = std::max(1, (4 * num_sms() + split_ctas - 1) / split_ctas);
   splits = (int)std::min<size_t>({(size_t)splits, (size_t)kMaxSplits,
                                   scratch_elems / (3 * (size_t)nb)});
   splits = std::max(1, splits);

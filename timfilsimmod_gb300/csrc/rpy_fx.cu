@@ -1,8 +1,8 @@
 // rpy_fx.cu -- the FP64 work-queue products, with the far-field pairs in
 // 64-bit fixed point (fx_pair.cuh).
 //
-// A product of FP64 jobs runs as two launches: fx_pack_kernel turns the packed
-// FP64 records into fixed-point ones and finds the scales; rpy_fx_kernel
+// A product of FP64 jobs runs as two launches: fx_pack_kernel packs the FP64
+// records, turns them into fixed-point ones and finds the scales; rpy_fx_kernel
 // computes the products. A job whose data the fixed-point form cannot take
 // (fx_pack_kernel's verdict, on the device: a swimmer more than 2^10 lambda
 // across, forces or positions that are not finite or outside 10^(+-270),
@@ -107,7 +107,8 @@ __device__ __forceinline__ i64 to_fixed(double v, int e) {
 
 // One thread per source of the two record arrays (segments first, each array
 // padded to whole tiles of 32 = one warp): fixed-point records and the tiles'
-// force exponents; the last CTA writes the sets' exponents and the verdict.
+// force exponents (and, from plain arrays, the FP64 records, which saves two
+// launches a product); the last CTA writes the sets' exponents and the verdict.
 // Latency bound; 45 FP64 instructions a thread made it 7.3 us, integer shifts
 // and FP32 norms in their place 7.1 us (4 876 particles): the atomics' round trips.
 __global__ void __launch_bounds__(kFxPackThreads) fx_pack_kernel(const FxSystem q) {
@@ -128,12 +129,24 @@ __global__ void __launch_bounds__(kFxPackThreads) fx_pack_kernel(const FxSystem 
   const bool warp_in = local * 32 < q.n[set], in = i < q.n[set];
   double f[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, x[3] = {0.0, 0.0, 0.0};
   if (in) {
-    const double *r = q.rec[set] + (size_t)i * len;
+    double *r = q.rec[set] + (size_t)i * len;
+    const bool raw = q.x[set] != nullptr;
+    const double *px = raw ? q.x[set] + 3 * (size_t)i : r;
+    const double *pf = raw ? q.f[set] + (size_t)fd * i : r + 3;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      x[k] = r[k];
-      f[k] = r[3 + k];
-      if (fd == 6) f[3 + k] = r[6 + k];
+      x[k] = px[k];
+      f[k] = pf[k];
+      if (fd == 6) f[3 + k] = pf[3 + k];
+    }
+    if (raw) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        r[k] = x[k];
+        r[3 + k] = f[k];
+        if (fd == 6) r[6 + k] = f[3 + k];
+      }
+      if (fd == 6) r[9] = 0.0;
     }
   }
   __syncthreads();

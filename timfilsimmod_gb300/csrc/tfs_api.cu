@@ -225,8 +225,8 @@ static QueueJob make_job(tfs_solver *s, bool tgt_segs, bool src_segs, bool src_b
 static void build_fx_systems(tfs_solver *s) {
   FxSystem &q = s->fx_sys;
   const double as = s->cfg.a_seg, ab = s->cfg.a_blob;
-  q.rec[0] = (const double *)s->rec_segs;
-  q.rec[1] = (const double *)s->rec_blobs;
+  q.rec[0] = (double *)s->rec_segs;
+  q.rec[1] = (double *)s->rec_blobs;
   q.n[0] = s->ns;
   q.n[1] = s->nb;
   q.fd[0] = 6;
@@ -296,16 +296,24 @@ int tfs::queue_product(tfs_solver *s, int list) {
   if ((fp32 || list < kNumQueueKinds) && (rc = ensure_origin(s)) != TFS_OK) return rc;
   // the records of both particle kinds: sources, and the targets' positions
   cudaError_t e;
-  if (s->ns > 0) {
-    e = launch_pack(fp32, 6, s->rec_segs, s->x_segs, s->f_segs, s->ns, s->origin, s->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "pack kernel");
+  if (!fp32 && list < kNumQueueKinds) {
+    FxSystem q = s->fx_sys;
+    q.x[0] = s->x_segs;
+    q.f[0] = s->f_segs;
+    q.x[1] = s->x_blobs;
+    q.f[1] = s->f_blobs;
+    if ((e = launch_fx_pack(q, s->stream)) != cudaSuccess)
+      return cuda_fail(e, "fixed-point pack kernel");
+  } else {
+    if (s->ns > 0) {
+      e = launch_pack(fp32, 6, s->rec_segs, s->x_segs, s->f_segs, s->ns, s->origin, s->stream);
+      if (e != cudaSuccess) return cuda_fail(e, "pack kernel");
+    }
+    if (s->nb > 0) {
+      e = launch_pack(fp32, 3, s->rec_blobs, s->x_blobs, s->f_blobs, s->nb, s->origin, s->stream);
+      if (e != cudaSuccess) return cuda_fail(e, "pack kernel");
+    }
   }
-  if (s->nb > 0) {
-    e = launch_pack(fp32, 3, s->rec_blobs, s->x_blobs, s->f_blobs, s->nb, s->origin, s->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "pack kernel");
-  }
-  if (!fp32 && list < kNumQueueKinds && (e = launch_fx_pack(s->fx_sys, s->stream)) != cudaSuccess)
-    return cuda_fail(e, "fixed-point pack kernel");
   if (s->product_service != nullptr)  // one launch shared with other swimmers' products
     return product_service_run(s->product_service, s, list, fp32, src);
   e = launch_queue(fp32, s->qtune[fp32][kind], src, s->qjobs_dev + 2 * list, s->qjobs[list],

@@ -100,7 +100,8 @@ struct FxState {
 constexpr int kFxEmpty = -100000;  // exponent of a set without forces
 // One particle system's records: [0] segments, [1] blobs (n = 0: none).
 struct FxSystem {
-  const double *rec[2];  // packed FP64 records
+  double *rec[2];        // packed FP64 records; written too where x is given
+  const double *x[2], *f[2];  // positions and forces [3 n], [fd n] to pack (null: rec holds them)
   long long *fx[2];      // fixed-point records: 9 (fd = 6) or 6 words each
   int *te[2];            // force exponents of the tiles of 32
   int n[2], fd[2];

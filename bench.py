@@ -362,10 +362,13 @@ def bench_ours(args):
                                          "velocities written (the written velocities and "
                                          "the chunk partial sums stay in L2)"},
             "fp64": {"value": value64, "unit": "matvecs/s", "steps": steps64,
-                     "roofline": {"bound": "fp64-fma", "achieved": achieved64,
+                     "roofline": {"bound": "integer-mad", "achieved": achieved64,
                                   "peak": peak64 / 1e12, "unit": "TFLOP/s",
                                   "frac": achieved64 / (peak64 / 1e12),
-                                  "avg_launch_ms": seg64_ms}},
+                                  "avg_launch_ms": seg64_ms,
+                                  "note": "FP64-accurate pairs in 64-bit fixed point on the "
+                                          "integer pipe: the FP64 FMA peak is the scale, "
+                                          "not the bound (fractions above 1)"}},
             "speedup_vs_fp64": value / value64,
             "rel_l2_error_vs_fp64": err,
             "clocks": clocks,
@@ -912,7 +915,7 @@ def large_bench(stream, flush, args, peak32, peak64):
         out[precision] = {"value": reps / (ms * 1e-3), "unit": "matvecs/s",
                           "ms_per_matvec": ms / reps, "reps": reps,
                           "pair_interactions_per_s": grand_pairs(ns, nb) * reps / (ms * 1e-3),
-                          "roofline": {"bound": f"{'fp32' if precision == 'fp32c' else 'fp64'}-fma",
+                          "roofline": {"bound": "fp32-fma" if precision == "fp32c" else "integer-mad",
                                        "achieved": achieved, "peak": peak / 1e12,
                                        "unit": "TFLOP/s", "frac": achieved / (peak / 1e12),
                                        "avg_launch_ms": launch_ms}}

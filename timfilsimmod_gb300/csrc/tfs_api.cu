@@ -305,14 +305,9 @@ int tfs::queue_product(tfs_solver *s, int list) {
     if ((e = launch_fx_pack(q, s->stream)) != cudaSuccess)
       return cuda_fail(e, "fixed-point pack kernel");
   } else {
-    if (s->ns > 0) {
-      e = launch_pack(fp32, 6, s->rec_segs, s->x_segs, s->f_segs, s->ns, s->origin, s->stream);
-      if (e != cudaSuccess) return cuda_fail(e, "pack kernel");
-    }
-    if (s->nb > 0) {
-      e = launch_pack(fp32, 3, s->rec_blobs, s->x_blobs, s->f_blobs, s->nb, s->origin, s->stream);
-      if (e != cudaSuccess) return cuda_fail(e, "pack kernel");
-    }
+    e = launch_pack_both(fp32, s->rec_segs, s->x_segs, s->f_segs, s->ns, s->rec_blobs, s->x_blobs,
+                         s->f_blobs, s->nb, s->origin, s->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "pack kernel");
   }
   if (s->product_service != nullptr)  // one launch shared with other swimmers' products
     return product_service_run(s->product_service, s, list, fp32, src);

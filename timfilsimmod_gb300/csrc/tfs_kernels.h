@@ -233,6 +233,10 @@ cudaError_t launch_pack(int fp32, int fd, void *rec, const double *x, const doub
                         const double *origin, cudaStream_t st);
 // FP32x2 records (positions negated, every value duplicated), 80 B per
 // segment and 48 B per blob.
+// The segments' and the blobs' records in one launch.
+cudaError_t launch_pack_both(int fp32, void *rec6, const double *x6, const double *f6, int n6,
+                             void *rec3, const double *x3, const double *f3, int n3,
+                             const double *origin, cudaStream_t st);
 cudaError_t launch_pack_x2(int fd, void *rec, const double *x, const double *f, int n,
                            const double *origin, cudaStream_t st);
 // vd: 6 (segment targets) or 3 (blob targets); fda/fdb: 6 (segment sources),

@@ -286,11 +286,8 @@ int tfs_flow_velocities(tfs_flow *f, double mu, int remove_net_force) {
   const int fp32 = f->precision == TFS_FP32C;
   const double *origin = fp32 ? f->origin : nullptr;  // FP64 records stay absolute
   cudaError_t e;
-  if (f->ns > 0 && (e = launch_pack(fp32, 6, f->rec_segs, f->x_segs, f->f_segs, f->ns, origin,
-                                    f->stream)) != cudaSuccess)
-    return cuda_fail(e, "pack kernel");
-  if (f->nb > 0 && (e = launch_pack(fp32, 3, f->rec_blobs, f->x_blobs, f->f_blobs, f->nb, origin,
-                                    f->stream)) != cudaSuccess)
+  if ((e = launch_pack_both(fp32, f->rec_segs, f->x_segs, f->f_segs, f->ns, f->rec_blobs,
+                            f->x_blobs, f->f_blobs, f->nb, origin, f->stream)) != cudaSuccess)
     return cuda_fail(e, "pack kernel");
   int n_points = f->nb;
   if (remove_net_force) {

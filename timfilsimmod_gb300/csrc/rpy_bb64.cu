@@ -133,6 +133,7 @@ __device__ __forceinline__ void plain_unit(const QueueJob &job, int grp, int c, 
   }
   __syncthreads();
   if (*s_last == 0) return;
+  static_assert(kChainBlock >= 6 * 32, "a thread per component of 32 targets");
   if (tid < VD * nb) {
     const double *p = part + (size_t)b0 * VD + tid;
     double r = 0.0;

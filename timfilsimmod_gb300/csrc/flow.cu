@@ -131,6 +131,10 @@ static cudaError_t launch_flow(FlowArgs a, int fp32, int wall, int variant, doub
   } else {
     a.mode = OUT_ASSIGN;
   }
+  // FP64: the integer products lengthen a warp's own chain of instructions, so
+  // they pay where an SM sub-partition has more than one warp (600 points, 262
+  // sources, 206 us without and 225 with; 2 000 points, 1 642 sources, 318 and 270)
+  a.soft = !fp32 && (long)ctas * splits * (var.block / 32) > 4L * num_sms();
   e = fn(a, dim3(ctas, splits), st, nullptr);
   count_launch();
   if (e != cudaSuccess) return e;

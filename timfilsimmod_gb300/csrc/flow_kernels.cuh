@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "rpy_pair2.cuh"
+#include "soft_mul.cuh"
 #include "rpy_tile.cuh"
 
 namespace tfs {
@@ -33,6 +34,7 @@ struct FlowArgs {
   double *out;             // 3 * n_flow, or split partials
   int mode;                // OUT_ASSIGN or OUT_PARTIAL
   int chunk;               // sources per split
+  int soft;                // FP64: products on the integer pipe
 };
 
 struct FlowVariant {
@@ -47,28 +49,34 @@ extern const FlowVariant g_flow_variants_f64[kFlowVariantsF64];
 extern const FlowFn g_flow_f32[kFlowVariantsF32][2];  // [variant][wall]
 extern const FlowFn g_flow_f64[kFlowVariantsF64][2];
 
-// v += sgn (rm1 f + rm3 (d.f) d): the Stokeslet of f at separation d
-template <typename T>
-__device__ __forceinline__ void stokeslet(T *v, T dx, T dy, T dz, T rm1, const T *f) {
-  const T rm3 = rm1 * rm1 * rm1;
-  const T w = rm3 * fma(dx, f[0], fma(dy, f[1], dz * f[2]));
+// The FP64 pairs. mul: how their plain products are formed -- on the integer
+// pipe (soft_mul.cuh), which runs beside the FP64 pipe that bounds this form: 10
+// of the 32 FP64 instructions of a segment source, 7 of 21 of a point's. The same
+// bits; 40 000 points around the medium swimmer 37.0 -> 25.6 ms, above the wall
+// (whose image terms stay as they are) 85.2 -> 78.7 ms.
+// v += rm1 f + rm3 (d.f) d: the Stokeslet of f at separation d
+template <typename T, typename Mul>
+__device__ __forceinline__ void stokeslet(T *v, T dx, T dy, T dz, const T *f, Mul mul) {
+  const T rm1 = rsqrt_far(fma(dx, dx, fma(dy, dy, mul(dz, dz))), mul);
+  const T rm3 = mul(mul(rm1, rm1), rm1);
+  const T w = mul(rm3, fma(dx, f[0], fma(dy, f[1], mul(dz, f[2]))));
   v[0] = fma(rm1, f[0], fma(w, dx, v[0]));
   v[1] = fma(rm1, f[1], fma(w, dy, v[1]));
   v[2] = fma(rm1, f[2], fma(w, dz, v[2]));
 }
 
 // One segment source: Stokeslet (Blakelet with WALL) + rotlet.
-template <typename T, bool WALL>
+template <typename T, bool WALL, typename Mul>
 __device__ __forceinline__ void flow_seg_pair(T *v, T xi, T yi, T zi, T sx, T sy, T sz,
-                                              const T *f) {
+                                              const T *f, Mul mul) {
   const T dx = xi - sx, dy = yi - sy, dz = zi - sz;
-  const T rm1 = rsqrt_far(fma(dx, dx, fma(dy, dy, dz * dz)));
-  const T rm3 = rm1 * rm1 * rm1;
-  const T w = rm3 * fma(dx, f[0], fma(dy, f[1], dz * f[2]));
+  const T rm1 = rsqrt_far(fma(dx, dx, fma(dy, dy, mul(dz, dz))), mul);
+  const T rm3 = mul(mul(rm1, rm1), rm1);
+  const T w = mul(rm3, fma(dx, f[0], fma(dy, f[1], mul(dz, f[2]))));
   // Stokeslet and rotlet (T x r) / r^3 (:118-123) share rm3
-  v[0] = fma(rm1, f[0], fma(w, dx, fma(rm3, f[4] * dz - f[5] * dy, v[0])));
-  v[1] = fma(rm1, f[1], fma(w, dy, fma(rm3, f[5] * dx - f[3] * dz, v[1])));
-  v[2] = fma(rm1, f[2], fma(w, dz, fma(rm3, f[3] * dy - f[4] * dx, v[2])));
+  v[0] = fma(rm1, f[0], fma(w, dx, fma(rm3, fma(f[4], dz, -mul(f[5], dy)), v[0])));
+  v[1] = fma(rm1, f[1], fma(w, dy, fma(rm3, fma(f[5], dx, -mul(f[3], dz)), v[1])));
+  v[2] = fma(rm1, f[2], fma(w, dz, fma(rm3, fma(f[3], dy, -mul(f[4], dx)), v[2])));
   if (WALL) {
     // minus the image Stokeslet at (sx, sy, -sz), then the source-doublet /
     // stresslet correction (:83-116); zi and sz are heights above the wall
@@ -194,7 +202,7 @@ __device__ __forceinline__ void flow_range2(const float (&xt)[TPT], const float 
   }
 }
 
-template <typename T, int FD, bool WALL, int BLOCK, int TPT, int TS>
+template <bool SOFT, typename T, int FD, bool WALL, int BLOCK, int TPT, int TS>
 __device__ __forceinline__ void flow_range(T (&v)[TPT][3], const T (&xt)[TPT], const T (&yt)[TPT],
                                            const T (&zt)[TPT], const T *__restrict__ rec, int lo,
                                            int hi, T *smem, float *hl) {
@@ -207,18 +215,28 @@ __device__ __forceinline__ void flow_range(T (&v)[TPT][3], const T (&xt)[TPT], c
     int4 *dst = reinterpret_cast<int4 *>(smem);
     for (int q = threadIdx.x; q < cnt * VEC_PER_REC; q += BLOCK) dst[q] = __ldg(src + q);
     __syncthreads();
-#pragma unroll 2
+#pragma unroll(SOFT ? 1 : 2)
     for (int j = 0; j < cnt; ++j) {
       T sx, sy, sz, f[FD];
       RecLoad<T, FD>::get(smem + j * L, sx, sy, sz, f);
 #pragma unroll
       for (int t = 0; t < TPT; ++t) {
-        if (FD == 6) {
-          flow_seg_pair<T, WALL>(v[t], xt[t], yt[t], zt[t], sx, sy, sz, f);
-        } else {
-          const T dx = xt[t] - sx, dy = yt[t] - sy, dz = zt[t] - sz;
-          stokeslet(v[t], dx, dy, dz, rsqrt_far(fma(dx, dx, fma(dy, dy, dz * dz))), f);
+        bool ok = true;
+        T u[3] = {v[t][0], v[t][1], v[t][2]};
+        auto pair = [&](auto mul) {
+          if constexpr (FD == 6)
+            flow_seg_pair<T, WALL>(u, xt[t], yt[t], zt[t], sx, sy, sz, f, mul);
+          else
+            stokeslet(u, xt[t] - sx, yt[t] - sy, zt[t] - sz, f, mul);
+        };
+        if constexpr (SOFT) pair([&](T a, T b) { return soft::mul(a, b, &ok); });
+        if (!SOFT || !ok) {  // (a point on a source, or numbers beyond the integer products)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) u[k] = v[t][k];
+          pair([](T a, T b) { return a * b; });
         }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[t][k] = u[k];
       }
     }
     Comp<T, 3, BLOCK, TPT>::fold(v, hl);
@@ -253,8 +271,11 @@ __global__ void __launch_bounds__(BLOCK) flow_kernel(const FlowArgs a) {
       if constexpr (kComp)
         flow_range2<6, WALL, BLOCK, TPT, TS>(
             xt, yt, zt, reinterpret_cast<const float *>(a.rec_segs), lo, hi, smem, hl);
+      else if (a.soft)
+        flow_range<true, T, 6, WALL, BLOCK, TPT, TS>(
+            v, xt, yt, zt, reinterpret_cast<const T *>(a.rec_segs), lo, hi, smem, hl);
       else
-        flow_range<T, 6, WALL, BLOCK, TPT, TS>(
+        flow_range<false, T, 6, WALL, BLOCK, TPT, TS>(
             v, xt, yt, zt, reinterpret_cast<const T *>(a.rec_segs), lo, hi, smem, hl);
     }
   }
@@ -264,8 +285,11 @@ __global__ void __launch_bounds__(BLOCK) flow_kernel(const FlowArgs a) {
       if constexpr (kComp)
         flow_range2<3, false, BLOCK, TPT, TS>(
             xt, yt, zt, reinterpret_cast<const float *>(a.rec_points), lo, hi, smem, hl);
+      else if (a.soft)
+        flow_range<true, T, 3, false, BLOCK, TPT, TS>(
+            v, xt, yt, zt, reinterpret_cast<const T *>(a.rec_points), lo, hi, smem, hl);
       else
-        flow_range<T, 3, false, BLOCK, TPT, TS>(
+        flow_range<false, T, 3, false, BLOCK, TPT, TS>(
             v, xt, yt, zt, reinterpret_cast<const T *>(a.rec_points), lo, hi, smem, hl);
     }
   }

@@ -66,9 +66,12 @@ TFS_FX Limb limb(u64 pb) { return {(int)(pb >> 32), (int)((unsigned)pb + 0x80000
 // words of P -> limbs of P
 TFS_FX Limb limb2(unsigned lo, unsigned hi) { return {(int)(hi + (lo >> 31)), (int)lo}; }
 TFS_FX Limb limb_of(i64 v) { return limb((u64)v + 0x80000000ull); }
-// Limbs whose low word is odd, so that both words can be negated: of P with
-// its truncation's half unit left out, which the odd low word makes up for.
-TFS_FX Limb odd_limb(u64 pb) { return {(int)(pb >> 32), (int)(((unsigned)pb ^ 0x80000000u) | 1u)}; }
+// Limbs that can be negated: the low word is not -2^31 (one place off where it
+// would be). Zero stays zero.
+TFS_FX Limb negatable(u64 pb) {
+  const int l = (int)((unsigned)pb ^ 0x80000000u);
+  return {(int)(pb >> 32), l > -0x7fffffff ? l : -0x7fffffff};
+}
 TFS_FX Limb minus(Limb a) { return {-a.h, -a.l}; }
 
 // a b + c: one IMAD.WIDE
@@ -251,16 +254,16 @@ TFS_FX bool far_pair(Acc *v, const u64 *x, const u64 *xs, const Limb *f, const L
 #pragma unroll
 #endif
     for (int k = 0; k < 3; ++k) {
-      xr[k] = odd_limb(madw(rho.h, w[k].h, mid_add(1ull << 63, rho, w[k]) >> 32));
+      xr[k] = negatable(madw(rho.h, w[k].h, mid_add(mid0<0>(), rho, w[k]) >> 32));
       xm[k] = minus(xr[k]);
     }
     if (FD == 6 && VD == 6) {
-      // 1/r^3: 2^-61, its truncation's half unit left out; a bias of any of
-      // the three would add up over sources with like torques
-      const u64 r3 = madw(r2.h, r1.h, mid_add(1ull << 63, r2, r1) >> 32) - 0x80000000ull;
-      h = minus(odd_limb((r3 >> 1) + 0x80000000ull));
+      // 1/r^3: 2^-61; a bias of any of the three would add up over sources with
+      // like torques
+      const u64 r3 = madw(r2.h, r1.h, mid_add(mid0<0>(), r2, r1) >> 32) - 0x80000000ull;
+      h = minus(negatable(((r3 + 1ull) >> 1) + 0x80000000ull));
       // 3/(2 r^3): 2^-63, below 0.61
-      p = mul<2>(mul<4>(limb(3ull * (2ull * r3 + 1ull) + 0x80000000ull), kappa), dot(w, t));
+      p = mul<2>(mul<4>(limb(6ull * r3 + 0x80000000ull), kappa), dot(w, t));
     }
   }
   // every addend's middle sums add 2^31 each to its bias

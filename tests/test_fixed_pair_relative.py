@@ -1,6 +1,14 @@
-"""The fixed-point far-field pair (csrc/fx_pair.cuh) keeps the exact zeros of
-configurations in a plane, as FP64 pairs do. The header compiled for the host,
-against the pair formula in long double. Tolerance: none."""
+"""The fixed-point far-field pair (csrc/fx_pair.cuh) keeps the relative accuracy
+of an FP64 pair at every distance, for each coupling by itself, and the exact
+zeros of configurations in a plane. The header compiled for the host, against
+the pair formula in long double.
+
+Tolerance: 2^-51 of the 2-norm of the pair's contribution, two last places of
+FP64. An FP64 pair is a chain of some eight roundings of 2^-53. In fixed point
+the factors of a coefficient and the coefficient itself are rounded to 2^-59 or
+finer against at least 1/8 (1/r^3 in [1/8, 1) of its power of two), the unit
+vector to 2^-62, and the reciprocal square root's series is cut at 2^-55: about
+ten errors of 2^-55."""
 import ctypes
 import os
 import subprocess
@@ -42,8 +50,8 @@ extern "C" void run(int fd, const double *x, const double *y, const double *f, i
       dF += d[k] * g[k];
       if (fd == 6) dT += d[k] * g[3 + k];
     }
-    if (fd == 6) PAIR6
-    else PAIR3
+    if (fd == 6) far_pair<6, 6>(v, xw, yw, F, T, pc, below[j]);
+    else far_pair<6, 3>(v, xw, yw, F, T, pc, below[j]);
     const Q r = sqrtl(r2), r3 = r * r2, r5 = r3 * r2;
     for (int k = 0; k < 3; ++k) {
       const int p = (k + 1) % 3, q = (k + 2) % 3;
@@ -67,12 +75,9 @@ extern "C" void run(int fd, const double *x, const double *y, const double *f, i
 '''
 
 
-def build(tmp, below):
-    arg = ", below[j]" if below else ""
-    text = SOURCE.replace("PAIR6", "far_pair<6, 6>(v, xw, yw, F, T, pc%s);" % arg).replace(
-        "PAIR3", "far_pair<6, 3>(v, xw, yw, F, T, pc%s);" % arg)
+def build(tmp):
     src, so = tmp / "fx.cpp", tmp / "fx.so"
-    src.write_text(text)
+    src.write_text(SOURCE)
     subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-std=c++17",
                     "-I", os.path.join(ROOT, "timfilsimmod_gb300", "csrc"), str(src),
                     "-o", str(so)], check=True, capture_output=True)
@@ -81,7 +86,7 @@ def build(tmp, below):
 
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
-    return build(tmp_path_factory.mktemp("fx"), False)
+    return build(tmp_path_factory.mktemp("fx"))
 
 
 def run(lib, fd, x, y, f, ex, es, a=1.0, below=None):
@@ -97,6 +102,39 @@ def run(lib, fd, x, y, f, ex, es, a=1.0, below=None):
 def frame(*xs):
     big = max(np.abs(x).max() for x in xs)
     return max(int(np.floor(np.log2(1.7320509 * big))) + 1, 1)
+
+
+@pytest.mark.parametrize("r", [2.0001, 2.9, 7.3, 50.0, 100.0, 300.0, 1000.0])
+@pytest.mark.parametrize("fd,kind", [(6, "force"), (6, "torque"), (3, "force")])
+def test_relative_error_of_a_pair(lib, r, fd, kind):
+    """One source with a force or a torque alone: the velocity and the angular
+    velocity each against their own size."""
+    rng = np.random.default_rng(int(10 * r))
+    for _ in range(200):
+        u, g = rng.normal(size=3), rng.normal(size=3)
+        u /= np.linalg.norm(u)
+        g /= np.linalg.norm(g) * (1 + 1e-6)
+        f = np.zeros((1, fd))
+        f[0, :3 if kind == "force" else 6][-3:] = g
+        x, y = 0.5 * r * u, -0.5 * r * u[None]
+        err, ref = run(lib, fd, x, y, f, frame(x, y), 0)
+        for part in (slice(0, 3), slice(3, 6)):
+            assert np.linalg.norm(err[part]) <= 2.0 ** -51 * np.linalg.norm(ref[part])
+
+
+@pytest.mark.parametrize("below", [1, 5, 9])
+@pytest.mark.parametrize("r", [2.2, 100.0])
+def test_a_source_below_the_largest(lib, r, below):
+    """A source 2^below smaller than the sums' unit has all its places."""
+    rng = np.random.default_rng(below)
+    for _ in range(100):
+        u, f = rng.normal(size=3), rng.normal(size=(1, 6))
+        u /= np.linalg.norm(u)
+        f *= 2.0 ** -below / np.linalg.norm(f) / (1 + 1e-6)
+        x, y = 0.5 * r * u, -0.5 * r * u[None]
+        err, ref = run(lib, 6, x, y, f, frame(x, y), 0, below=[below])
+        for part in (slice(0, 3), slice(3, 6)):
+            assert np.linalg.norm(err[part]) <= 2.0 ** -51 * np.linalg.norm(ref[part])
 
 
 @pytest.mark.parametrize("fd", [6, 3])

@@ -1404,8 +1404,8 @@ int pres_alloc(tfs_solver *s) {
            "cudaHostAlloc");
   if ((rc = alloc_dev((void **)&p->fx_rec[0], 48 * ns)) != TFS_OK ||
       (rc = alloc_dev((void **)&p->fx_rec[1], 48 * nb)) != TFS_OK ||
-      (rc = alloc_dev((void **)&p->fx_te[0], sizeof(int) * ((ns + 31) / 32))) != TFS_OK ||
-      (rc = alloc_dev((void **)&p->fx_te[1], sizeof(int) * ((nb + 31) / 32))) != TFS_OK ||
+      (rc = alloc_dev((void **)&p->fx_te[0], sizeof(int) * ns)) != TFS_OK ||
+      (rc = alloc_dev((void **)&p->fx_te[1], sizeof(int) * nb)) != TFS_OK ||
       (rc = alloc_dev((void **)&p->fx_state, sizeof(FxState))) != TFS_OK)
     return rc;
   {

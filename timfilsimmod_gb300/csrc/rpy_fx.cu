@@ -12,7 +12,7 @@
 //
 // rpy_fx_kernel. Work units, persistent CTAs, arrival counters and the
 // determinism argument are rpy_queue.cuh's. A fixed-point unit's chunk is a
-// run of tiles of 32 sources; the chunk sums are kept as 96-bit integers of one
+// run of tiles of 32 sources; the chunk sums are kept as 128-bit integers of one
 // scale per job, so the last unit of a target block adds the chunks exactly
 // and converts once to FP64. Pairs at or inside contact (itself, touching or
 // overlapping particles), which the fixed-point pair leaves out and reports
@@ -21,13 +21,16 @@
 // their unit.
 //
 // Bound: issue of the integer multiply-adds (IMAD.WIDE, two cycles each) and
-// of the carry additions and shifts between them: 450 instructions a 6x6 pair,
-// 840 cycles a warp and SM sub-partition, against 52 FP64 instructions of 78
-// cycles. Occupancy does not matter (3, 4 and 5 CTAs of 128 an SM within 3%).
-// Medium swimmer (12 800 segments, 2 562 blobs), before and after: M_ss 9.19
-// and 3.72 ms, M_bs 1.38 and 0.56, M_sb 1.38 and 0.51, M_bb 0.36 and 0.10. The
-// error against 64-bit sums is not larger: 2-norm over the velocities 1.5e-15
-// against 1.9e-15 (both with the 64-bit sums' own).
+// of the carry additions and shifts between them: some 970 cycles a 6x6 pair,
+// warp and SM sub-partition, against 52 FP64 instructions of 78 cycles.
+// Occupancy does not matter (3 and 4 CTAs of 128 an SM within 2%).
+// Medium swimmer (12 800 segments, 2 562 blobs), FP64 sums and these: M_ss 9.19
+// and 4.30 ms, M_bs 1.38 and 0.79, M_sb 1.38 and 0.60, M_bb 0.36 and 0.11. (M_ss
+// 3.72, M_bs 0.56, M_sb 0.51 ms with coefficients of a fixed place, whose error
+// grows with the distance: fx_pair.cuh.) The error against 64-bit sums is not
+// larger, neither in the 2-norm over all velocities (1.5e-15 against 1.9e-15,
+// both with the 64-bit sums' own) nor for a target alone, far from the loaded
+// particles or with forces far below the largest.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -106,8 +109,8 @@ __device__ __forceinline__ i64 to_fixed(double v, int e) {
 }
 
 // One thread per source of the two record arrays (segments first, each array
-// padded to whole tiles of 32 = one warp): fixed-point records and the tiles'
-// force exponents (and, from plain arrays, the FP64 records, which saves two
+// padded to whole warps): fixed-point records, each source's force with an
+// exponent of its own (and, from plain arrays, the FP64 records, which saves two
 // launches a product); the last CTA writes the sets' exponents and the verdict.
 // Latency bound; 45 FP64 instructions a thread made it 7.3 us, integer shifts
 // and FP32 norms in their place 7.1 us (4 876 particles): the atomics' round trips.
@@ -183,13 +186,12 @@ __global__ void __launch_bounds__(kFxPackThreads) fx_pack_kernel(const FxSystem 
       }
     }
     bad = bad && in;
+    int top = e;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
     if (bad) atomicOr(&s_bad, 1);
-    if (lane == 0) {
-      q.te[set][local] = e;
-      atomicMax(&s_es[set], e);
-    }
+    if (lane == 0) atomicMax(&s_es[set], top);
+    if (in) q.te[set][i] = e;
     if (in && !bad) {
       i64 *w = q.fx[set] + (size_t)i * (fd == 6 ? 9 : 6);
 #pragma unroll
@@ -249,20 +251,47 @@ __device__ __noinline__ void exact_pair(double *v, const double *xt, const doubl
   rpy_pair<double, VD, FD>(v, dx, dy, dz, f, c);
 }
 
-__device__ __forceinline__ void acc_add_signed(Acc &a, i64 v) {
-  const unsigned s = (unsigned)(v >> 63);
-  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
-      : "+r"(a.w1), "+r"(a.w2), "+r"(a.w3)
-      : "r"((unsigned)v), "r"((unsigned)((u64)v >> 32)), "r"(s));
+__device__ __forceinline__ void add128(unsigned (&a)[4], unsigned b0, unsigned b1, unsigned b2,
+                                       unsigned b3) {
+  asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\t"
+      "addc.u32 %3, %3, %7;"
+      : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3])
+      : "r"(b0), "r"(b1), "r"(b2), "r"(b3));
+}
+
+// a += round(v 2^e), |v 2^e| < 2^95, by integer shifts as to_fixed.
+__device__ __forceinline__ void acc_add_fixed(Acc &a, double v, int e) {
+  const u64 b = (u64)__double_as_longlong(v);
+  const int ev = (int)(b >> 52) & 0x7ff;
+  const int s = min(ev - 1075 + e, 63);
+  const u64 m = ev == 0 ? 0ull : (b & 0xfffffffffffffull) | (1ull << 52);
+  u64 lo = 0ull, hi = 0ull;
+  if (s >= 0) {
+    lo = m << s;
+    hi = s > 0 ? m >> (64 - s) : 0ull;
+  } else if (s >= -60) {
+    lo = (m + (1ull << (-s - 1))) >> -s;
+  }
+  if ((i64)b < 0) {
+    lo = 0ull - lo;
+    hi = ~hi + (lo == 0ull ? 1ull : 0ull);
+  }
+  unsigned w[4] = {a.w0, a.w1, a.w2, a.w3};
+  add128(w, fx::low(lo), fx::high(lo), fx::low(hi), fx::high(hi));
+  a.w0 = w[0];
+  a.w1 = w[1];
+  a.w2 = w[2];
+  a.w3 = w[3];
 }
 
 constexpr int kFp64Tile = 128;  // sources per staged tile of the FP64 units (fixes their sums' order)
 
 // 16-byte aligned records of a staged source: position words, force limbs,
-// torque limbs.
+// torque limbs, the exponent below the job's.
 template <int FD>
 struct Staged {
-  static constexpr int words = FD == 6 ? 20 : 12;  // 32-bit
+  static constexpr int words = FD == 6 ? 20 : 16;  // 32-bit
+  static constexpr int below = FD == 6 ? 18 : 12;
 };
 
 __device__ __forceinline__ Limb shifted(i64 v, int s) {
@@ -284,16 +313,21 @@ __device__ __forceinline__ void sum_tiles(Acc (&v)[VD], const u64 (&xt)[3], cons
   pc.shift = Ex - src.lx;
   pc.s = src.s;
   pc.near_q = src.near_q * __int_as_float((127 + 58 - 2 * pc.shift) << 23);
-  const double up = pow2(59 - es + src.lx);  // v -> integer: 2^59 lambda / 2^es
-  const double upr = pow2(59 - es + 2 * src.lx);
+  const int up = 91 - es + src.lx;  // v -> integer: 2^91 lambda / 2^es
   const int s1 = min(t1 * 32, n);
   for (int base = t0 * 32; base < s1; base += TS) {
     const int cnt = min(TS, s1 - base);
     __syncthreads();
     for (int j = threadIdx.x; j < cnt; j += BLOCK) {
       const i64 *w = src.rec + (size_t)(base + j) * (FD == 6 ? 9 : 6);
-      const int sh = min(es - src.te[(base + j) >> 5], 63);
+      // a source up to 2^kMaxBelow smaller than the job's largest keeps all its
+      // places (the pair shifts its sums); below, the places that are lost are
+      // 2^-71 of the largest
+      const int es_below = es - src.te[base + j];
+      const int below = min(es_below, (int)fx::kMaxBelow);
+      const int sh = min(es_below - below, 63);
       const int sht = min(sh + src.tshift, 63);
+      smem[j * W + Staged<FD>::below] = (unsigned)below;
       u64 *o = reinterpret_cast<u64 *>(smem + j * W);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -327,7 +361,8 @@ __device__ __forceinline__ void sum_tiles(Acc (&v)[VD], const u64 (&xt)[3], cons
           t[1] = {(int)(d.y >> 32), (int)d.y};
           t[2] = {(int)(e >> 32), (int)e};
         }
-        if (fx::far_pair<VD, FD>(v, xt, xs, f, t, pc)) near |= 1u << j;
+        const unsigned below = smem[(sub + j) * W + Staged<FD>::below];
+        if (fx::far_pair<VD, FD>(v, xt, xs, f, t, pc, below)) near |= 1u << j;
       }
       while (near) {
         const int j = __ffs(near) - 1;
@@ -336,16 +371,16 @@ __device__ __forceinline__ void sum_tiles(Acc (&v)[VD], const u64 (&xt)[3], cons
         exact_pair<VD, FD>(u, tgt, rec + (size_t)(base + sub + j) * (FD == 6 ? 10 : 6),
                            job.pc64[set]);
 #pragma unroll
-        for (int k = 0; k < VD; ++k)
-          acc_add_signed(v[k], __double2ll_rn(u[k] * (k < 3 ? up : upr)));
+        for (int k = 0; k < VD; ++k) acc_add_fixed(v[k], u[k], k < 3 ? up : up + src.lx);
       }
     }
     count += (unsigned)cnt;
   }
 }
 
-struct Sum96 {
-  unsigned w[3];
+// A chunk's sum, signed, unit 2^-91.
+struct __align__(16) Sum128 {
+  unsigned w[4];
 };
 
 template <int VD, int FDA, int FDB, int BLOCK>
@@ -378,8 +413,8 @@ __device__ __forceinline__ void fx_unit(const QueueJob &job, int blk, int c, uns
       sum_tiles<VD, FDB, BLOCK>(v, xt, tgt, job, 1, max(t0 - ta, 0), t1 - ta, es, Ex, smem, active,
                                 count);
   }
-  // the sums without their biases, unit 2^-59
-  Sum96 sum[VD];
+  // the sums without their biases
+  Sum128 sum[VD];
 #pragma unroll
   for (int k = 0; k < VD; ++k) {
     // count (2^62 + 2^31) off the upper 96 bits
@@ -387,15 +422,18 @@ __device__ __forceinline__ void fx_unit(const QueueJob &job, int blk, int c, uns
     const unsigned top = (unsigned)(count >> 2) + (b1 < b0 ? 1u : 0u);
     u64 lo = fx::pack64(v[k].w1, v[k].w2);
     const u64 l = lo - b1;
-    sum[k].w[0] = (unsigned)l;
-    sum[k].w[1] = (unsigned)(l >> 32);
-    sum[k].w[2] = v[k].w3 - top - (lo < b1 ? 1u : 0u);
+    sum[k].w[0] = v[k].w0;
+    sum[k].w[1] = (unsigned)l;
+    sum[k].w[2] = (unsigned)(l >> 32);
+    sum[k].w[3] = v[k].w3 - top - (lo < b1 ? 1u : 0u);
   }
   if (job.fx_chunks > 1) {
-    Sum96 *p = reinterpret_cast<Sum96 *>(job.partial);
+    uint4 *p = reinterpret_cast<uint4 *>(job.partial);
     if (i0 < n_tgt) {
 #pragma unroll
-      for (int k = 0; k < VD; ++k) p[((size_t)c * VD + k) * n_tgt + i0] = sum[k];
+      for (int k = 0; k < VD; ++k)
+        p[((size_t)c * VD + k) * n_tgt + i0] =
+            make_uint4(sum[k].w[0], sum[k].w[1], sum[k].w[2], sum[k].w[3]);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -407,16 +445,13 @@ __device__ __forceinline__ void fx_unit(const QueueJob &job, int blk, int c, uns
     if (*s_last == 0) return;
     if (threadIdx.x == 0) job.block_done[blk] = 0u;
 #pragma unroll
-    for (int k = 0; k < VD; ++k) sum[k].w[0] = sum[k].w[1] = sum[k].w[2] = 0u;
+    for (int k = 0; k < VD; ++k) sum[k].w[0] = sum[k].w[1] = sum[k].w[2] = sum[k].w[3] = 0u;
 #pragma unroll 4
     for (int cc = 0; cc < job.fx_chunks; ++cc) {
 #pragma unroll
       for (int k = 0; k < VD; ++k) {
-        const unsigned *w = p[((size_t)cc * VD + k) * n_tgt + i].w;
-        const unsigned a = __ldcg(w), b = __ldcg(w + 1), d = __ldcg(w + 2);
-        asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
-            : "+r"(sum[k].w[0]), "+r"(sum[k].w[1]), "+r"(sum[k].w[2])
-            : "r"(a), "r"(b), "r"(d));
+        const uint4 a = __ldcg(p + ((size_t)cc * VD + k) * n_tgt + i);
+        add128(sum[k].w, a.x, a.y, a.z, a.w);
       }
     }
   }
@@ -425,9 +460,15 @@ __device__ __forceinline__ void fx_unit(const QueueJob &job, int blk, int c, uns
   double *o = job.out + (size_t)i0 * VD;
 #pragma unroll
   for (int k = 0; k < VD; ++k) {
-    const i64 top = (i64)fx::pack64(sum[k].w[1], sum[k].w[2]);
-    const double val = fma((double)top, 4294967296.0, (double)sum[k].w[0]);
-    const double r = val * pow2(es - 59 - (k < 3 ? lx : 2 * lx)) * job.scale;
+    u64 top = fx::pack64(sum[k].w[2], sum[k].w[3]), bot = fx::pack64(sum[k].w[0], sum[k].w[1]);
+    const bool minus = (i64)top < 0;
+    if (minus) {
+      bot = 0ull - bot;
+      top = ~top + (bot == 0ull ? 1ull : 0ull);
+    }
+    const double mag = fma((double)top, 18446744073709551616.0, (double)bot);
+    const double val = minus ? -mag : mag;
+    const double r = val * pow2(es - 91 - (k < 3 ? lx : 2 * lx)) * job.scale;
     o[k] = job.mode == OUT_ACCUMULATE ? o[k] + r : r;
   }
 }

@@ -419,8 +419,8 @@ int tfs_solver_create(const tfs_config *cfg, tfs_solver **out) {
       (rc = alloc_dev(&s->rec_blobs_x2, 48 * (size_t)nb)) ||
       (rc = alloc_dev((void **)&s->fx_rec[0], 72 * (size_t)ns)) ||
       (rc = alloc_dev((void **)&s->fx_rec[1], 48 * (size_t)nb)) ||
-      (rc = alloc_dev((void **)&s->fx_te[0], sizeof(int) * ((size_t)(ns + 31) / 32))) ||
-      (rc = alloc_dev((void **)&s->fx_te[1], sizeof(int) * ((size_t)(nb + 31) / 32))) ||
+      (rc = alloc_dev((void **)&s->fx_te[0], sizeof(int) * (size_t)ns)) ||
+      (rc = alloc_dev((void **)&s->fx_te[1], sizeof(int) * (size_t)nb)) ||
       (rc = alloc_dev((void **)&s->fx_state, sizeof(FxState))) ||
       (rc = alloc_dev(&s->rec_ff, ff_record_bytes() * nb)) ||
       (rc = alloc_dev(&s->bar_grid, barrier_grid_bytes(ns, nb))) ||
@@ -998,6 +998,6 @@ size_t solver_bytes_estimate(const tfs_config *cfg) {
   const size_t n = 3 * nb + 6, m = std::min<size_t>(350, n);
   const size_t doubles = 15 * ns + 12 * nb + (size_t)kMaxSplits * (6 * ns + 3 * nb) +
                          n * (m + 1) + (m + 1) * (m + 1) + 16 * n + 57 * nb + 256 * (m + 1);
-  return 8 * doubles + 273 * ns + 249 * nb + ((size_t)1 << 20);
+  return 8 * doubles + 276 * ns + 252 * nb + ((size_t)1 << 20);
 }
 }  // namespace tfs

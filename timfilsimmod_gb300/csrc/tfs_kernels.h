@@ -103,7 +103,7 @@ struct FxSystem {
   double *rec[2];        // packed FP64 records; written too where x is given
   const double *x[2], *f[2];  // positions and forces [3 n], [fd n] to pack (null: rec holds them)
   long long *fx[2];      // fixed-point records: 9 (fd = 6) or 6 words each
-  int *te[2];            // force exponents of the tiles of 32
+  int *te[2];            // force exponents of the sources
   int n[2], fd[2];
   const double *origin;  // the origin kernel's result
   int lx_min, lx_max;    // of lambda over the pair kinds
@@ -118,9 +118,9 @@ struct FxSource {
   float near_q;    // (a_i + a_j)^2 / lambda^2, widened
   fx::Limb s;
 };
-// At most this many chunks: their 12-byte partial sums fit where kMaxSplits
-// 8-byte ones do.
-constexpr int kFxMaxChunks = kMaxSplits * 8 / 12;
+// At most this many chunks: their 16-byte partial sums fit where kMaxSplits
+// 8-byte ones do (and start on 16 bytes: kMaxSplits is even).
+constexpr int kFxMaxChunks = kMaxSplits * 8 / 16;
 
 struct QueueJob {
   const void *tgt_rec;     // packed records of the targets (their positions are read)

@@ -3,6 +3,8 @@ result is far below that of the largest force over lambda."""
 import numpy as np
 import pytest
 
+from oracle import Oracle
+
 pytestmark = pytest.mark.gpu
 Q = np.longdouble
 
@@ -132,3 +134,29 @@ def test_small_forces_beside_a_large_one():
                             (ss[i, 3:], vr, fs[i, 3:] / k)):
             size = np.sqrt((v**2).sum(-1)).sum() + np.linalg.norm(own)
             assert np.linalg.norm((got - (v.sum(0) + own)).astype(float)) <= TOL * size
+
+
+@pytest.mark.parametrize("length,force", [(1e14, 1e-264), (1e-14, 1e258), (1e14, 1e258),
+                                          (1e-14, 1e-258), (1e5, 1e-238), (1e-5, 1e240)])
+def test_exponents_of_lengths_and_forces(length, force):
+    """Lengths and forces whose exponents add up; the bar of every FP64 product."""
+    from timfilsimmod_gb300.mobility import RpyMobilitySolver
+
+    rng = np.random.default_rng(1)
+    x = 2.5 * np.stack(np.meshgrid(*[np.arange(4.0)] * 3), -1).reshape(-1, 3)
+    f = rng.normal(size=(64, 6))
+    f[:, 3:] *= length  # F L and T of a size
+    s = RpyMobilitySolver(1, 64, 1, 0, "fp64", a_seg=length, a_blob=length)
+    s.set_state(length * x, force * f, np.zeros((0, 3)), np.zeros((0, 3)))
+    s.evaluate_segment_segment_mobility()
+    s.copy_segment_velocities_to_host()
+    s.wait_for_device()
+    got = s.v_segs_host.reshape(-1, 6).copy()
+    s.finalise()
+    f[:, 3:] /= length
+    want = Oracle(1.0, 1.0, 1.0).mss(x, f).reshape(-1, 6)
+    got[:, :3] *= length
+    got[:, 3:] *= length
+    got[:, 3:] *= length
+    got = got / force
+    assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))

@@ -5,7 +5,7 @@
 // records, turns them into fixed-point ones and finds the scales; rpy_fx_kernel
 // computes the products. A job whose data the fixed-point form cannot take
 // (fx_pack_kernel's verdict, on the device: a swimmer more than 2^10 lambda
-// across, forces or positions that are not finite or outside 10^(+-270),
+// across, forces or positions that are not finite or outside 2^(+-kFxExponent),
 // positions outside the frame the origin kernel last saw; or radii too far
 // apart for one lambda, known on the host) runs on the FP64 pipe instead, as
 // units of rpy_queue.cuh in the same launch.
@@ -53,6 +53,11 @@ using fx::u64;
 
 constexpr int kFxPackThreads = 256;
 constexpr int kNoForce = kFxEmpty;
+// Forces up to 2^(+-kFxExponent) and lambda up to 2^(+-kFxLambda): an exponent es of
+// a force, or of a torque over lambda, is then within kFxExponent + kFxLambda + 1, and
+// the results' factor 2^(es - 91 - 2 lx) within 2^(+-1000). Beyond, FP64 sums.
+constexpr int kFxExponent = 800, kFxLambda = 20;
+static_assert(kFxExponent + 3 * kFxLambda + 1 + 91 <= 1000, "pow2's range");
 
 // The frame of a product: positions relative to o in units of 2^(Ex - 61).
 struct Frame {
@@ -172,7 +177,7 @@ __global__ void __launch_bounds__(kFxPackThreads) fx_pack_kernel(const FxSystem 
         if (v != 0.0) e0 = max(e0, exponent_of(v));
       }
       if (e0 > kNoForce) {
-        bad = bad || e0 > 896 || e0 < -896;  // and infinities, NaN, subnormals
+        bad = bad || e0 > kFxExponent || e0 < -kFxExponent;  // and infinities, NaN, subnormals
         if (!bad) {
           // the norm of the components over 2^e0, in FP32 (relative error 2^-21)
           float n2 = 0.f;
@@ -576,7 +581,7 @@ bool fx_job(QueueJob *j, FxState *state, const long long *tgt, const FxSource &a
   const double ra = j->a_a, rb = j->n_b > 0 ? j->a_b : j->a_a;
   // one lambda per job, of its smaller contact distance
   const int lx = fx_lambda_exponent(j->a_tgt, std::min(ra, rb));
-  if (std::abs(lx) > 60 || std::abs(lx_min) > 60) return false;
+  if (std::abs(lx) > kFxLambda || std::abs(lx_min) > kFxLambda) return false;
   for (int set = 0; set < 2; ++set) {
     const double at = ldexp(j->a_tgt, -lx), as = ldexp(set == 0 ? ra : rb, -lx);
     FxSource &f = j->fx[set];

@@ -332,7 +332,10 @@ int tfs_prescribed_set_solution(tfs_solver *s, const double *f_segs, const doubl
 int tfs_solver_autotune(tfs_solver *s, int precision_mask, int reps);
 /* Pin the work-queue variant of one product kind: kind 0..5 = M_ss, M_bs,
  * M_ss with M_bs, M_sb, M_bb, grand mobility; variant in
- * [0, tfs_num_queue_variants(precision)). */
+ * [0, tfs_num_queue_variants(precision)). FP64 products that keep one order of
+ * their sums (solves and implicit steps) take one kernel at every size, whatever
+ * autotune picks; a variant other than 0, pinned here, keeps them in the tile
+ * form, which gives the same bits. */
 int tfs_solver_set_queue_variant(tfs_solver *s, int precision, int kind, int variant);
 int tfs_num_queue_variants(int precision);
 /* Pin the launch of one combination: combo 0..5 = seg<-seg, seg<-blob,

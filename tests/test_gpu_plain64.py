@@ -68,3 +68,34 @@ def test_step_products(nfil, nseg):
         out.append({k: np.array(g[k]) for k in ("x", "q", "body_x", "body_q", "tether")})
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k]) and np.array_equal(out[0][k], out[2][k]), k
+
+
+def test_autotuned_solver_keeps_the_plain_kernel():
+    """Autotuning times the kernels of the fixed-point form; what it picks leaves
+    the plain products alone."""
+    torch = pytest.importorskip("torch")
+    from torch.profiler import ProfilerActivity, profile
+
+    from timfilsimmod_gb300.geometry import elastic_swimmer
+    from timfilsimmod_gb300.mobility import RpyMobilitySolver
+    from timfilsimmod_gb300.stepper import ImplicitStepper
+
+    for nfil in range(5, 13):
+        blob_refs, fil_refs, fil_dirs, radius = elastic_swimmer(nfil, 11, 2.2)
+        s = RpyMobilitySolver(1, nfil, 11, len(blob_refs), "fp64", end_force_magnitude=220)
+        s.set_blob_references(blob_refs)
+        s.set_linear_solver(1e-8)
+        st = ImplicitStepper(s, nfil, 11, fil_refs, fil_dirs, seg_sep=2.2, dt=1e-3, tol=1e-4,
+                             end_force_magnitude=220, body_radius=radius)
+        st.step(0)
+        s.autotune(("fp64",), reps=1)
+        for nt in (1, 2):  # (the first trace of a process may be empty)
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                st.step(nt)
+                torch.cuda.synchronize()
+        names = " ".join(e.name for e in prof.events())
+        if "arnoldi" not in names:
+            pytest.skip("no kernel trace")
+        assert "rpy_plain64_kernel" in names and "rpy_fx_kernel" not in names, nfil
+        st.close()
+        s.finalise()

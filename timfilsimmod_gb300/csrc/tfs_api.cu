@@ -311,8 +311,12 @@ int tfs::queue_product(tfs_solver *s, int list) {
   }
   if (s->product_service != nullptr)  // one launch shared with other swimmers' products
     return product_service_run(s->product_service, s, list, fp32, src);
-  e = launch_queue(fp32, s->qtune[fp32][kind], src, s->qjobs_dev + 2 * list, s->qjobs[list],
-                   s->qjobs_n[list], s->qcount, s->stream, next_events(s));
+  // the tuned variants are of the other form's kernels: plain FP64 products have
+  // one form that is the fastest at every size, and the tile form for a caller
+  // who pins a variant
+  const int variant = list < kNumQueueKinds ? s->qtune[fp32][kind] : s->plain_tile[kind] ? 1 : 0;
+  e = launch_queue(fp32, variant, src, s->qjobs_dev + 2 * list, s->qjobs[list], s->qjobs_n[list],
+                   s->qcount, s->stream, next_events(s));
   if (e != cudaSuccess) return cuda_fail(e, "RPY work-queue kernel");
   return TFS_OK;
 }
@@ -960,6 +964,7 @@ int tfs_solver_set_queue_variant(tfs_solver *s, int precision, int kind, int var
   if (variant < 0 || variant >= tfs_num_queue_variants(precision))
     return fail(TFS_EINVAL, "variant %d out of range", variant);
   s->qtune[precision][kind] = variant;
+  if (precision == TFS_FP64) s->plain_tile[kind] = variant != 0;
   return TFS_OK;
 }
 

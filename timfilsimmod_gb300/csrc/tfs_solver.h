@@ -114,6 +114,7 @@ struct tfs_solver {
   tfs::QueueJob *qjobs_dev = nullptr;  // [kNumQueueLists][2]
   unsigned *qcount = nullptr;          // [2] launch counters, then arrival counters
   int qtune[2][tfs::kNumQueueKinds] = {};
+  bool plain_tile[tfs::kNumQueueKinds] = {};  // FP64 plain products kept in the tile form
   // products shared with other swimmers' (one work-queue launch for all that
   // are waiting): the service, and events marking this swimmer's records
   // ready and its product done

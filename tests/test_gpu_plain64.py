@@ -99,3 +99,40 @@ def test_autotuned_solver_keeps_the_plain_kernel():
         assert "rpy_plain64_kernel" in names and "rpy_fx_kernel" not in names, nfil
         st.close()
         s.finalise()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32c"])
+@pytest.mark.parametrize("nfil,nseg", [(4, 10), (19, 17)])
+def test_a_broyden_loop_of_the_caller_gets_the_stepper_s_velocities(precision, nfil, nseg):
+    """compute_velocities through the public call, as a program with a Broyden loop
+    of its own makes it, and inside the library's implicit step."""
+    from timfilsimmod_gb300.geometry import elastic_swimmer
+    from timfilsimmod_gb300.mobility import RpyMobilitySolver
+    from timfilsimmod_gb300.stepper import ImplicitStepper
+
+    blob_refs, fil_refs, fil_dirs, radius = elastic_swimmer(nfil, nseg, 2.2)
+    u0 = 1e-3 * np.random.default_rng(nfil).normal(size=3 * nfil * nseg)
+    out = []
+    for public in (False, True):
+        s = RpyMobilitySolver(1, nfil, nseg, len(blob_refs), precision, end_force_magnitude=220)
+        s.set_blob_references(blob_refs)
+        s.set_linear_solver(1e-8)
+        st = ImplicitStepper(s, nfil, nseg, fil_refs, fil_dirs, seg_sep=2.2, dt=1e-3, tol=1e-4,
+                             end_force_magnitude=220, body_radius=radius)
+        st.reset(u0)
+        st.initial_guess(0)
+        f = st.forces_and_torques(0)
+        if public:
+            g = st.state()
+            s.set_body_pose(g["body_x"], g["body_q"])
+            s.positions_updated()
+            s.compute_velocities(f)
+        else:
+            st.compute_velocities(0)
+        s.copy_segment_velocities_to_host()
+        s.wait_for_device()
+        out.append([s.v_segs_host.copy(), s.blob_forces().copy(), s.body_velocities().copy()])
+        st.close()
+        s.finalise()
+    for a, b in zip(*out):
+        assert np.any(a != 0.0) and np.array_equal(a, b)

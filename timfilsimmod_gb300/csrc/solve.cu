@@ -1046,7 +1046,7 @@ namespace tfs {
 // (s->swimmer_f, updated in place with the blob repulsion's sums as the
 // reference updates swimmer::f): queued on s->stream with one host wait per
 // refinement cycle and none at the end.
-int compute_velocities_dev(tfs_solver *s, int *gmres_iters, bool step) {
+int compute_velocities_dev(tfs_solver *s, int *gmres_iters) {
   if (s->cfg.nswim != 1) return fail(TFS_EINVAL, "compute_velocities solves one swimmer per solver");
   if (!s->have_refs) return fail(TFS_ESTATE, "set the blob references first");
   int rc;
@@ -1059,18 +1059,9 @@ int compute_velocities_dev(tfs_solver *s, int *gmres_iters, bool step) {
                      s->service == nullptr && s->product_service == nullptr;
   if (early && (rc = early_residual_product(s)) != TFS_OK) return rc;
   // v_segs = Mss f_segs, v_blobs = Mbs f_segs (one work-queue launch when
-  // both target sets exist)
+  // both target sets exist), in the plain form (build_queue_jobs)
   if (s->ns > 0 && s->nb > 0) {
-    if (step) {
-      rc = queue_product(s, QL_SEGSRC_PLAIN);
-    } else {
-      // M_ss, then M_bs in the plain form (build_queue_jobs). FP64: one launch
-      // of both forms would take longer (1 264 against 1 041 us at 3 587 segments
-      // and 1 289 blobs: an FP64 instruction holds the issue port).
-      if ((rc = queue_product(s, QK_MSS)) != TFS_OK) return rc;
-      rc = queue_product(s, QL_MBS_PLAIN);
-    }
-    if (rc != TFS_OK) return rc;
+    if ((rc = queue_product(s, QL_SEGSRC_PLAIN)) != TFS_OK) return rc;
   } else {
     if ((rc = tfs_evaluate_segment_segment_mobility(s)) != TFS_OK) return rc;
     if ((rc = tfs_evaluate_blob_segment_mobility(s)) != TFS_OK) return rc;
@@ -1082,7 +1073,7 @@ int compute_velocities_dev(tfs_solver *s, int *gmres_iters, bool step) {
   int iters = 0;
   if ((rc = linear_solve(s, &iters, early)) != TFS_OK) return rc;
   // v_segs += Msb f_blobs (the solved blob forces)
-  if (step && s->pres == nullptr && s->ns > 0 && s->nb > 0)
+  if (s->pres == nullptr && s->ns > 0 && s->nb > 0)
     rc = queue_product(s, QL_MSB_PLAIN);
   else
     rc = tfs_evaluate_segment_blob_mobility(s);
@@ -1128,7 +1119,7 @@ int tfs_compute_velocities(tfs_solver *s, double *swimmer_f, int *gmres_iters) {
   std::memcpy(s->f6_host, swimmer_f, 8 * 6);
   TFS_CUDA(cudaMemcpyAsync(s->swimmer_f, s->f6_host, 8 * 6, cudaMemcpyHostToDevice, s->stream),
            "copy swimmer force");
-  int rc = compute_velocities_dev(s, gmres_iters, false);
+  int rc = compute_velocities_dev(s, gmres_iters);
   if (rc != TFS_OK) return rc;
   TFS_CUDA(cudaMemcpyAsync(s->f6_host, s->swimmer_f, 8 * 6, cudaMemcpyDeviceToHost, s->stream),
            "read swimmer force");

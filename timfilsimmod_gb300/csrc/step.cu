@@ -1596,7 +1596,7 @@ int stepper_velocities(tfs_stepper *st, int *gmres_iters) {
   int rc = tfs_set_body_pose(st->s, st->bx, st->bq);
   if (rc != TFS_OK) return rc;
   st->s->origin_dirty = true;
-  return tfs::compute_velocities_dev(st->s, gmres_iters, true);
+  return tfs::compute_velocities_dev(st->s, gmres_iters);
 }
 
 }  // namespace

@@ -259,15 +259,15 @@ static int build_queue_jobs(tfs_solver *s) {
   add_job(s, QK_MBB, false, false, true, OUT_ASSIGN);
   add_job(s, QK_GRAND, true, true, true, OUT_ASSIGN);
   add_job(s, QK_GRAND, false, true, true, OUT_ASSIGN);
-  // Sums whose rounding the caller's iteration amplifies keep the plain form.
-  // FP64: the right-hand side of the free-body solve, M_bs (a difference of
-  // 1e-14 in a warm start grows up to 1e5 times in the solution of the FP64
-  // GMRES), and every product of an implicit step (Broyden's iteration carries
-  // 1e-15 in a velocity to 1e-9 in the tether forces). FP32C the same: 4e-7 in
-  // M_bs is up to 2e-5 in the blob forces, and a swimmer's displacement over a
-  // step is a small difference of its filaments'.
-  static const int plain_lists[3][2] = {
-      {QK_MBS, QL_MBS_PLAIN}, {QK_SEGSRC, QL_SEGSRC_PLAIN}, {QK_MSB, QL_MSB_PLAIN}};
+  // Sums whose rounding an iteration around them amplifies keep the plain form:
+  // the products of compute_velocities, the library's own implicit step or a
+  // caller's Broyden loop around the public call. FP64: a difference of 1e-14 in
+  // the right-hand side's M_bs grows up to 1e5 times in a warm-started GMRES
+  // solution, and Broyden's iteration carries 1e-15 in a velocity to 1e-9 in the
+  // tether forces. FP32C the same: 4e-7 in M_bs is up to 2e-5 in the blob forces,
+  // and a swimmer's displacement over a step is a small difference of its
+  // filaments'.
+  static const int plain_lists[2][2] = {{QK_SEGSRC, QL_SEGSRC_PLAIN}, {QK_MSB, QL_MSB_PLAIN}};
   for (const auto &l : plain_lists) {
     s->qjobs_n[l[1]] = s->qjobs_n[l[0]];
     for (int j = 0; j < s->qjobs_n[l[0]]; ++j) {
@@ -287,10 +287,9 @@ static int queue_sources(int kind) {
 
 int tfs::queue_product(tfs_solver *s, int list) {
   const int fp32 = s->cfg.precision == TFS_FP32C;
-  const int kind = list < kNumQueueKinds ? list
-                   : list == QL_MBS_PLAIN ? (int)QK_MBS
+  const int kind = list < kNumQueueKinds  ? list
                    : list == QL_MSB_PLAIN ? (int)QK_MSB
-                                         : (int)QK_SEGSRC;
+                                          : (int)QK_SEGSRC;
   const int src = queue_sources(kind);
   int rc;
   if ((fp32 || list < kNumQueueKinds) && (rc = ensure_origin(s)) != TFS_OK) return rc;
@@ -314,7 +313,8 @@ int tfs::queue_product(tfs_solver *s, int list) {
   // the tuned variants are of the other form's kernels: plain FP64 products have
   // one form that is the fastest at every size, and the tile form for a caller
   // who pins a variant
-  const int variant = list < kNumQueueKinds ? s->qtune[fp32][kind] : s->plain_tile[kind] ? 1 : 0;
+  const bool tile = s->plain_tile[kind] || (kind == QK_SEGSRC && s->plain_tile[QK_MBS]);
+  const int variant = list < kNumQueueKinds ? s->qtune[fp32][kind] : tile ? 1 : 0;
   e = launch_queue(fp32, variant, src, s->qjobs_dev + 2 * list, s->qjobs[list], s->qjobs_n[list],
                    s->qcount, s->stream, next_events(s));
   if (e != cudaSuccess) return cuda_fail(e, "RPY work-queue kernel");

@@ -210,8 +210,8 @@ long long queue_units(const QueueJob *jobs_host, int n_jobs, int block_targets);
 enum QueueKind { QK_MSS = 0, QK_MBS = 1, QK_SEGSRC = 2, QK_MSB = 3, QK_MBB = 4, QK_GRAND = 5 };
 constexpr int kNumQueueKinds = 6;
 // The same lists with their jobs in the plain form (QueueJob::plain).
-constexpr int kNumQueueLists = 9;
-enum { QL_MBS_PLAIN = 6, QL_SEGSRC_PLAIN = 7, QL_MSB_PLAIN = 8 };
+constexpr int kNumQueueLists = 8;
+enum { QL_SEGSRC_PLAIN = 6, QL_MSB_PLAIN = 7 };
 
 // Tuning of one launch: variant and the number of full waves (resident CTAs
 // on every SM) the source splitting aims for.

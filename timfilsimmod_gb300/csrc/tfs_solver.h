@@ -184,8 +184,7 @@ int product_service_run(ProductService *sv, tfs_solver *s, int list, int fp32, i
 void product_service_stats(ProductService *sv, long long *launches, long long *products);
 // compute_velocities on the swimmer force already in s->swimmer_f, queued on
 // s->stream without a host wait at the end (solve.cu).
-// step: the call is part of an implicit step.
-int compute_velocities_dev(tfs_solver *s, int *gmres_iters, bool step);
+int compute_velocities_dev(tfs_solver *s, int *gmres_iters);
 // A new time step begins (the stepper's initial guess): FP32C solvers keep
 // the last step's final solution for the extrapolated warm start of the next
 // step's first solve (solve.cu).

@@ -16,6 +16,7 @@
 #include <condition_variable>
 #include <chrono>
 
+#include "flights.h"
 #include "tfs_solver.h"
 
 using namespace tfs;
@@ -373,15 +374,12 @@ struct GmresService {
   };
   static constexpr int kSlots = 8;
   static constexpr size_t kInFlight = 4;  // launches at once
+  static_assert(kInFlight < kSlots, "a free slot for the next launch");
   struct Slot {
     PgArgs *args = nullptr, *dev_args = nullptr;  // launch arguments, host staging and device
     int2 *map = nullptr, *dev_map = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t copied = nullptr, done = nullptr;
-  };
-  struct Flight {  // a launch that may still run
-    cudaEvent_t done;
-    int ctas;
   };
   std::mutex m;
   std::condition_variable cv;
@@ -389,39 +387,13 @@ struct GmresService {
   bool busy = false;
   int sms = 1;
   Slot slot[kSlots];
-  int next_slot = 0;
-  std::deque<Flight> flights;  // oldest first
+  Flights flights;
   long long launches = 0, solves = 0;
 
-  // CTAs in flight (ended launches leave the list).
+  // CTAs in flight.
   int in_flight() {
-    int used = 0;
-    for (auto it = flights.begin(); it != flights.end();) {
-      if (cudaEventQuery(it->done) == cudaErrorNotReady) {
-        used += it->ctas;
-        ++it;
-      } else {
-        it = flights.erase(it);
-      }
-    }
-    return used;
-  }
-
-  // The next slot; st follows the launch that its event stood for.
-  int take_slot(Slot **out, cudaStream_t st) {
-    Slot &sl = slot[next_slot];
-    next_slot = (next_slot + 1) % kSlots;
-    if (st == nullptr) st = sl.stream;
-    for (auto it = flights.begin(); it != flights.end();) {
-      if (it->done == sl.done) {
-        TFS_CUDA(cudaStreamWaitEvent(st, sl.done, 0), "service: wait for the slot");
-        it = flights.erase(it);
-      } else {
-        ++it;
-      }
-    }
-    *out = &sl;
-    return TFS_OK;
+    return flights.ctas(
+        [&](int s) { return cudaEventQuery(slot[s].done) != cudaErrorNotReady; });
   }
 
   // Queues one launch of the solves in batch (the leader, without the lock;
@@ -470,7 +442,7 @@ struct GmresService {
       busy = true;
       int used;
       while ((used = in_flight()) > 0 &&
-             (flights.size() >= kInFlight || used + pending.front()->args.P > sms))
+             (flights.list.size() >= kInFlight || used + pending.front()->args.P > sms))
         cv.wait_for(g, std::chrono::microseconds(20));
       std::vector<Req *> batch;
       int ctas = 0;
@@ -480,13 +452,12 @@ struct GmresService {
         batch.push_back(pending.front());
         pending.pop_front();
       }
-      Slot *sl = nullptr;
-      int lrc = take_slot(&sl, nullptr);
+      const int sl = flights.free_slot(kSlots);
       g.unlock();
-      if (lrc == TFS_OK) lrc = launch(batch, *sl);
+      const int lrc = launch(batch, slot[sl]);
       g.lock();
       if (lrc == TFS_OK) {
-        flights.push_back({sl->done, ctas});
+        flights.add(sl, ctas);
         ++launches;
         solves += (long long)batch.size();
       }
@@ -506,15 +477,14 @@ struct GmresService {
   int own_launch(tfs_solver *s, F launch_it) {
     std::unique_lock<std::mutex> g(m);
     cv.wait(g, [&] { return !busy; });
-    Slot *sl = nullptr;
-    int rc = take_slot(&sl, s->stream);
-    if (rc != TFS_OK) return rc;
-    for (const Flight &f : flights)
-      TFS_CUDA(cudaStreamWaitEvent(s->stream, f.done, 0), "service: wait for CTAs");
-    flights.clear();
+    int rc;
+    const int sl = flights.free_slot(kSlots);
+    for (const Flights::Flight &f : flights.list)
+      TFS_CUDA(cudaStreamWaitEvent(s->stream, slot[f.slot].done, 0), "service: wait for CTAs");
+    flights.list.clear();
     if ((rc = launch_it()) != TFS_OK) return rc;
-    TFS_CUDA(cudaEventRecord(sl->done, s->stream), "service: completion");
-    flights.push_back({sl->done, sms});
+    TFS_CUDA(cudaEventRecord(slot[sl].done, s->stream), "service: completion");
+    flights.add(sl, sms);
     return TFS_OK;
   }
 };

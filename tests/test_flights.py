@@ -25,6 +25,14 @@ int fly(int n, int ctas, long end) {
   f.add(s, ctas);
   return s;
 }
+// which call fails: 0 none, 1 the wait for a flight, 2 the launch, 3 the record
+int alone(int n, int ctas, int fails, int *waits, int *synced) {
+  *waits = *synced = 0;
+  return f.alone(f.free_slot(n), ctas, [&](int) { ++*waits; return fails == 1 ? -1 : 0; },
+                 [&] { return fails == 2 ? -2 : 0; },
+                 [&](int s) { ends[s] = now + 50; return fails == 3 ? -3 : 0; },
+                 [&] { *synced = 1; });
+}
 }
 '''
 
@@ -62,3 +70,19 @@ def test_slots_are_of_one_launch_each(lib):
     lib.wait_until(12)  # three have ended
     assert lib.ctas() == 5
     assert sorted(lib.fly(8, 1, 50) for _ in range(3)) == [0, 1, 2]
+
+
+@pytest.mark.parametrize("fails", [0, 1, 2, 3])
+def test_a_launch_on_all_ctas(lib, fails):
+    """It replaces the flights it waits for, unless a step of it fails: then they
+    stay, and a launch whose end is not recorded is waited for."""
+    lib.reset()
+    for k in range(3):
+        lib.fly(8, 10, 20)
+    waits, synced = ctypes.c_int(), ctypes.c_int()
+    rc = lib.alone(8, 152, fails, ctypes.byref(waits), ctypes.byref(synced))
+    assert rc == -fails and waits.value == (1 if fails == 1 else 3)
+    assert synced.value == (fails == 3)
+    assert lib.ctas() == (152 if fails == 0 else 30)
+    lib.wait_until(20)
+    assert lib.ctas() == (152 if fails == 0 else 0)

@@ -41,6 +41,24 @@ struct Flights {
   }
 
   void add(int slot, int ctas) { list.push_back({slot, ctas}); }
+
+  // A launch of ctas CTAs behind every flight, in the given slot: wait(slot) for
+  // each, launch(), record(slot), each 0 or an error that ends it. Only a launch
+  // whose end is recorded replaces the flights; one that is not is synchronised.
+  template <typename Wait, typename Launch, typename Record, typename Sync>
+  int alone(int slot, int ctas, Wait wait, Launch launch, Record record, Sync sync) {
+    int rc;
+    for (const Flight &f : list)
+      if ((rc = wait(f.slot)) != 0) return rc;
+    if ((rc = launch()) != 0) return rc;
+    if ((rc = record(slot)) != 0) {
+      sync();
+      return rc;
+    }
+    list.clear();
+    add(slot, ctas);
+    return 0;
+  }
 };
 
 }  // namespace tfs

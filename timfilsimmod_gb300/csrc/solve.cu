@@ -455,6 +455,7 @@ struct GmresService {
       const int sl = flights.free_slot(kSlots);
       g.unlock();
       const int lrc = launch(batch, slot[sl]);
+      if (lrc != TFS_OK) cudaStreamSynchronize(slot[sl].stream);  // nothing uncounted runs on
       g.lock();
       if (lrc == TFS_OK) {
         flights.add(sl, ctas);
@@ -477,15 +478,18 @@ struct GmresService {
   int own_launch(tfs_solver *s, F launch_it) {
     std::unique_lock<std::mutex> g(m);
     cv.wait(g, [&] { return !busy; });
-    int rc;
-    const int sl = flights.free_slot(kSlots);
-    for (const Flights::Flight &f : flights.list)
-      TFS_CUDA(cudaStreamWaitEvent(s->stream, slot[f.slot].done, 0), "service: wait for CTAs");
-    flights.list.clear();
-    if ((rc = launch_it()) != TFS_OK) return rc;
-    TFS_CUDA(cudaEventRecord(slot[sl].done, s->stream), "service: completion");
-    flights.add(sl, sms);
-    return TFS_OK;
+    return flights.alone(
+        flights.free_slot(kSlots), sms,
+        [&](int k) -> int {
+          TFS_CUDA(cudaStreamWaitEvent(s->stream, slot[k].done, 0), "service: wait for CTAs");
+          return TFS_OK;
+        },
+        launch_it,
+        [&](int k) -> int {
+          TFS_CUDA(cudaEventRecord(slot[k].done, s->stream), "service: completion");
+          return TFS_OK;
+        },
+        [&] { cudaStreamSynchronize(s->stream); });
   }
 };
 

@@ -79,7 +79,8 @@ int tfs_solver_destroy(tfs_solver *s);
 /* Run the solver's work on `stream` (a cudaStream_t; NULL = the solver's own
  * non-blocking stream). */
 int tfs_solver_set_stream(tfs_solver *s, void *stream);
-/* Change the pairwise-sum arithmetic (TFS_FP64 / TFS_FP32C). */
+/* Change the pairwise-sum arithmetic (TFS_FP64 / TFS_FP32C). A solver created as
+ * FP32C allocates the FP64 products' records the first time it becomes FP64. */
 int tfs_solver_set_precision(tfs_solver *s, int precision);
 
 /* Device buffers of the solver (AoS float64), for callers that keep data

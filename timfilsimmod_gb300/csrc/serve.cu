@@ -332,7 +332,7 @@ int tfs_server::build(Instance *in, const tfs_request &r) {
   int rc = tfs_config_default(&c, 1, r.nfil, r.nseg, r.nblob);
   if (rc != TFS_OK) return rc;
   c.precision = cfg.precision;
-  if ((rc = tfs_solver_create(&c, &in->s)) != TFS_OK) return rc;
+  if ((rc = tfs::solver_create(&c, false, &in->s)) != TFS_OK) return rc;
   if ((rc = tfs_set_linear_solver(in->s, cfg.linear_tol, std::min(350, 3 * r.nblob + 6))) != TFS_OK)
     return rc;
   if (cfg.precision == TFS_FP32C) {

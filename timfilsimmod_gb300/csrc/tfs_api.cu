@@ -86,6 +86,17 @@ static cudaEvent_t *next_events(tfs_solver *s) {
   return p;
 }
 
+static void fx_free(tfs_solver *s) {
+  for (int k = 0; k < 2; ++k) {
+    cudaFree(s->fx_rec[k]);
+    cudaFree(s->fx_te[k]);
+    s->fx_rec[k] = nullptr;
+    s->fx_te[k] = nullptr;
+  }
+  cudaFree(s->fx_state);
+  s->fx_state = nullptr;
+}
+
 static void free_all(tfs_solver *s) {
   for (cudaEvent_t e : s->events) cudaEventDestroy(e);
   s->events.clear();
@@ -106,11 +117,7 @@ static void free_all(tfs_solver *s) {
   cudaFree(s->rec_blobs);
   cudaFree(s->rec_segs_x2);
   cudaFree(s->rec_blobs_x2);
-  for (int k = 0; k < 2; ++k) {
-    cudaFree(s->fx_rec[k]);
-    cudaFree(s->fx_te[k]);
-  }
-  cudaFree(s->fx_state);
+  fx_free(s);
   cudaFree(s->rec_ff);
   cudaFree(s->bar_grid);
   cudaFree(s->wc_z);
@@ -281,6 +288,35 @@ static int build_queue_jobs(tfs_solver *s) {
   return TFS_OK;
 }
 
+// The fixed-point records and scales of FP64 block products (76 bytes a segment,
+// 52 a blob), and the job lists with them. FP32C solvers, and the solvers of a
+// server, whose products are FP32 or plain, do without: allocated at creation,
+// with the precision FP64 set later, or (in a server) on first use.
+static int ensure_fx(tfs_solver *s) {
+  if (s->fx_state != nullptr) return TFS_OK;
+  int rc;
+  const FxState fx0{0, 0, {kFxEmpty, kFxEmpty}, 0, {kFxEmpty, kFxEmpty}, 0u};
+  // (launches under way read the job lists)
+  TFS_CUDA(cudaStreamSynchronize(s->stream), "fixed-point records");
+  if ((rc = alloc_dev((void **)&s->fx_rec[0], 72 * (size_t)s->ns)) ||
+      (rc = alloc_dev((void **)&s->fx_rec[1], 48 * (size_t)s->nb)) ||
+      (rc = alloc_dev((void **)&s->fx_te[0], sizeof(int) * (size_t)s->ns)) ||
+      (rc = alloc_dev((void **)&s->fx_te[1], sizeof(int) * (size_t)s->nb)) ||
+      (rc = alloc_dev((void **)&s->fx_state, sizeof fx0))) {
+    fx_free(s);
+    return rc;
+  }
+  cudaError_t e = cudaMemcpy(s->fx_state, &fx0, sizeof fx0, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    build_fx_systems(s);
+    if ((rc = build_queue_jobs(s)) == TFS_OK) return TFS_OK;
+  } else {
+    rc = cuda_fail(e, "fixed-point state");
+  }
+  fx_free(s);
+  return rc;
+}
+
 static int queue_sources(int kind) {
   return kind == QK_GRAND ? Q_SEG_BLOB : (kind == QK_MSB || kind == QK_MBB) ? Q_BLOB : Q_SEG;
 }
@@ -296,6 +332,7 @@ int tfs::queue_product(tfs_solver *s, int list) {
   // the records of both particle kinds: sources, and the targets' positions
   cudaError_t e;
   if (!fp32 && list < kNumQueueKinds) {
+    if ((rc = ensure_fx(s)) != TFS_OK) return rc;
     FxSystem q = s->fx_sys;
     q.x[0] = s->x_segs;
     q.f[0] = s->f_segs;
@@ -365,6 +402,12 @@ int tfs_config_default(tfs_config *cfg, int nswim, int nfil, int nseg, int nblob
 }
 
 int tfs_solver_create(const tfs_config *cfg, tfs_solver **out) {
+  return tfs::solver_create(cfg, true, out);
+}
+
+}  // extern "C"
+
+int tfs::solver_create(const tfs_config *cfg, bool blocks, tfs_solver **out) {
   if (cfg == nullptr || out == nullptr) return fail(TFS_EINVAL, "null argument");
   *out = nullptr;
   if (cfg->nswim < 0 || cfg->nfil < 0 || cfg->nseg < 0 || cfg->nblob < 0)
@@ -421,11 +464,6 @@ int tfs_solver_create(const tfs_config *cfg, tfs_solver **out) {
       (rc = alloc_dev(&s->rec_blobs, record_bytes(0, 3) * nb)) ||
       (rc = alloc_dev(&s->rec_segs_x2, 80 * (size_t)ns)) ||
       (rc = alloc_dev(&s->rec_blobs_x2, 48 * (size_t)nb)) ||
-      (rc = alloc_dev((void **)&s->fx_rec[0], 72 * (size_t)ns)) ||
-      (rc = alloc_dev((void **)&s->fx_rec[1], 48 * (size_t)nb)) ||
-      (rc = alloc_dev((void **)&s->fx_te[0], sizeof(int) * (size_t)ns)) ||
-      (rc = alloc_dev((void **)&s->fx_te[1], sizeof(int) * (size_t)nb)) ||
-      (rc = alloc_dev((void **)&s->fx_state, sizeof(FxState))) ||
       (rc = alloc_dev(&s->rec_ff, ff_record_bytes() * nb)) ||
       (rc = alloc_dev(&s->bar_grid, barrier_grid_bytes(ns, nb))) ||
       (rc = alloc_dev((void **)&s->scratch, dsz * s->scratch_elems)) ||
@@ -452,11 +490,10 @@ int tfs_solver_create(const tfs_config *cfg, tfs_solver **out) {
   cudaMemsetAsync(s->origin, 0, dsz * origin_elems(), s->stream);
   cudaMemsetAsync(s->origin_cnt, 0, 2 * sizeof(unsigned), s->stream);
   cudaMemsetAsync(s->qcount, 0, sizeof(unsigned) * qcount_elems, s->stream);
-  const FxState fx0{0, 0, {kFxEmpty, kFxEmpty}, 0, {kFxEmpty, kFxEmpty}, 0u};
-  cudaMemcpyAsync(s->fx_state, &fx0, sizeof fx0, cudaMemcpyHostToDevice, s->stream);
   e = cudaStreamSynchronize(s->stream);
   build_fx_systems(s);
-  if (e == cudaSuccess && (rc = build_queue_jobs(s)) != TFS_OK) {
+  if (e == cudaSuccess &&
+      (rc = blocks && cfg->precision == TFS_FP64 ? ensure_fx(s) : build_queue_jobs(s)) != TFS_OK) {
     free_all(s);
     delete s;
     return rc;
@@ -469,6 +506,8 @@ int tfs_solver_create(const tfs_config *cfg, tfs_solver **out) {
   *out = s;
   return TFS_OK;
 }
+
+extern "C" {
 
 int tfs_solver_destroy(tfs_solver *s) {
   if (s == nullptr) return TFS_OK;
@@ -488,6 +527,10 @@ int tfs_solver_set_precision(tfs_solver *s, int precision) {
   TFS_CHECK_SOLVER(s);
   if (precision != TFS_FP64 && precision != TFS_FP32C)
     return fail(TFS_EINVAL, "unknown precision %d", precision);
+  if (precision == TFS_FP64) {
+    const int rc = ensure_fx(s);
+    if (rc != TFS_OK) return rc;
+  }
   s->cfg.precision = precision;
   return TFS_OK;
 }
@@ -795,6 +838,7 @@ int tfs_solver_autotune(tfs_solver *s, int precision_mask, int reps) {
     if (s->ns > 0 && (rc = pack(s, 1)) != TFS_OK) break;
     if (s->nb > 0 && (rc = pack(s, 0)) != TFS_OK) break;
     if (p == TFS_FP64) {
+      if ((rc = ensure_fx(s)) != TFS_OK) break;
       const cudaError_t pe = launch_fx_pack(s->fx_sys, s->stream);
       if (pe != cudaSuccess) {
         rc = cuda_fail(pe, "fixed-point pack kernel");
@@ -995,7 +1039,7 @@ long long tfs_kernel_launch_count(void) { return g_launches.load(); }
 }  // extern "C"
 
 namespace tfs {
-// Device bytes of a solver of these sizes (tfs_solver_create's and the
+// Device bytes of a server's solver of these sizes (solver_create's and the
 // solve's allocations, the cooperative-GMRES buffers at their largest),
 // plus 1 MB for the small ones.
 size_t solver_bytes_estimate(const tfs_config *cfg) {
@@ -1003,6 +1047,6 @@ size_t solver_bytes_estimate(const tfs_config *cfg) {
   const size_t n = 3 * nb + 6, m = std::min<size_t>(350, n);
   const size_t doubles = 15 * ns + 12 * nb + (size_t)kMaxSplits * (6 * ns + 3 * nb) +
                          n * (m + 1) + (m + 1) * (m + 1) + 16 * n + 57 * nb + 256 * (m + 1);
-  return 8 * doubles + 276 * ns + 252 * nb + ((size_t)1 << 20);
+  return 8 * doubles + 200 * ns + 200 * nb + ((size_t)1 << 20);
 }
 }  // namespace tfs

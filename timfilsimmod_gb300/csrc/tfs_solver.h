@@ -168,6 +168,9 @@ int queue_product(tfs_solver *s, int list);
 int h2d_f32(tfs_solver *s, double *dst, const float *src, size_t n, const char *what);
 int d2h_f32(tfs_solver *s, float *dst, const double *src, size_t n, const char *what);
 int alloc_dev(void **p, size_t bytes);
+// tfs_solver_create. blocks: the caller may launch single block products and the
+// grand mobility, under capture too, so an FP64 solver has all they need.
+int solver_create(const tfs_config *cfg, bool blocks, tfs_solver **out);
 int solve_alloc(tfs_solver *s);
 void solve_free(tfs_solver *s);
 // Inner solves of FP32C swimmers batched into shared cooperative launches.

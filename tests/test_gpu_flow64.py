@@ -35,3 +35,26 @@ def test_same_as_alone(nseg, nblob, zero):
         out.append(e.v_flow_host.reshape(-1, 3)[:100].copy())
         e.close()
     assert np.abs(out[0] - out[1]).max() <= 1e-12 * np.abs(out[1]).max()
+
+
+@pytest.mark.parametrize("nseg,nblob", [(1, 0), (100, 0), (63, 5), (70, 57), (1, 126)])
+def test_same_bits_with_one_split(nseg, nblob):
+    """Fewer than 128 sources are one split whatever the points: the same points
+    with and without the integer products, bit for bit."""
+    from timfilsimmod_gb300.flow_field import FlowFieldEvaluator
+
+    rng = np.random.default_rng(nseg + nblob)
+    xs, fs = rng.uniform(-20, 20, (nseg, 3)), rng.normal(size=(nseg, 6))
+    xb, fb = rng.uniform(-20, 20, (nblob, 3)), rng.normal(size=(nblob, 3))
+    xs[:, 2] += 25.0
+    fs[::2, 1:5] = 0.0
+    many = rng.uniform(-30, 30, (80000, 3)) + (0.0, 0.0, 31.0)
+    out = []
+    for p in (many, many[:100]):
+        e = FlowFieldEvaluator(1, nseg, 1, nblob, len(p), precision="fp64")
+        e.read_positions_and_forces(p, xs, fs, xb, fb, np.zeros(3))
+        e.velocities()
+        e.wait()
+        out.append(e.v_flow_host.reshape(-1, 3)[:100].copy())
+        e.close()
+    assert np.any(out[0] != 0.0) and np.array_equal(out[0], out[1])

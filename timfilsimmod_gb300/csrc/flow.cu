@@ -132,8 +132,10 @@ static cudaError_t launch_flow(FlowArgs a, int fp32, int wall, int variant, doub
     a.mode = OUT_ASSIGN;
   }
   // FP64: the integer products lengthen a warp's own chain of instructions, so
-  // they pay where an SM sub-partition has more than one warp (600 points, 262
-  // sources, 206 us without and 225 with; 2 000 points, 1 642 sources, 318 and 270)
+  // they pay where an SM sub-partition has more than one warp. 300 to 40 000 points,
+  // 262 to 4 876 sources, with a wall and without: on one warp 9 to 15% slower (262
+  // sources, up to 8 000 points: 205 us without and 230 with), on two and more 4 to
+  // 30% faster (2 000 points, 1 642 sources: 308 and 273; 16 000: 1 578 and 1 130)
   a.soft = !fp32 && (long)ctas * splits * (var.block / 32) > 4L * num_sms();
   e = fn(a, dim3(ctas, splits), st, nullptr);
   count_launch();

@@ -9,7 +9,9 @@
 namespace tfs {
 
 // Units of 128 targets that a product is cut into where there is work enough,
-// and about as many as are resident at once (four to five CTAs on each SM).
+// and about as many as a GB300 runs at once (152 SMs of four to five CTAs).
+// Constants, not the launch's own occupancy: the chunks fix the order of the sums,
+// and a product's bits depend on its sizes alone, not on the variant that runs it.
 constexpr long kUnits = 8192, kQueueFill = 700;
 
 void queue_chunking(int n_src, int n_particles, int *chunk, int *n_chunks) {

@@ -210,7 +210,10 @@ int tfs_set_body_reference_matrices(tfs_solver *s, const double *body_mobility,
  * swimmer_f holds F with the blob repulsion added, as the reference leaves
  * swimmer.f; segment velocities, blob forces and body velocity are on the
  * device (tfs_copy_segment_velocities_to_host, tfs_copy_blob_forces_to_host,
- * tfs_get_body_velocities). Synchronises the solver's stream. */
+ * tfs_get_body_velocities). The products keep one order of plain sums, the same
+ * here and in tfs_stepper_step, as a Broyden loop around the call amplifies their
+ * rounding; the block hooks above take the faster forms. Synchronises the
+ * solver's stream. */
 int tfs_compute_velocities(tfs_solver *s, double *swimmer_f, int *gmres_iters);
 /* The linear solve alone (solve_linear_system, mobility_solver.cpp:2092-2570)
  * for a right-hand side rhs_host[3 nblob + 6]. */

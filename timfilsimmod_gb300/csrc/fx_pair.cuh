@@ -19,8 +19,8 @@
 // every sum below stays under 2^63 with the sizes written beside it.
 //
 // Scales. Lengths are measured in lambda = 2^lx, the largest power of two
-// below 0.74 (a_i + a_j) (fx_lx): lambda/r and s/r^2 stay under 1. Positions
-// are round((x - o) 2^(61 - Ex)), |x - o| < 2^Ex (FxFrame); a source's force
+// below 0.74 (a_i + a_j) (fx_lambda_exponent): lambda/r and s/r^2 stay under 1. Positions
+// are round((x - o) 2^(61 - Ex)), |x - o| < 2^Ex (frame_of); a source's force
 // and torque are round(F 2^(62 - es + below)), |F| <= 2^(es - below), |T| <=
 // lambda 2^(es - below), es the exponent of the job's largest.
 //

@@ -587,7 +587,8 @@ bool fx_job(QueueJob *j, FxState *state, const long long *tgt, const FxSource &a
     FxSource &f = j->fx[set];
     f.lx = lx;
     f.tshift = lx - lx_min;
-    // widened by 2^-18: the FP32 r^2 it is compared with is within 2^-20
+    // widened by 2^-18: the FP32 r^2 it is compared with is within 2^-18.6 (at
+    // contact in the widest frame, where the separation's words have 21 bits)
     f.near_q = (float)((at + as) * (at + as) * (1.0 + 3.8147e-6));
     const double sq = (at * at + as * as) / 3.0;
     if (!(sq < 3.9)) return false;  // radii too far apart for one lambda
